@@ -1,12 +1,14 @@
 // devtest.cu - C-ABI harness around the public device functions of include/csmv_tx.cuh, built as
 // lib/libcsmv_devtest.so so the GPU tests can pin each function against the CPU oracle on
-// arbitrary inputs: the version read rule, TXPreValidation, TXWriteBack's slot choice, and the
-// bounded wait that turns a wait nobody satisfies into an error status instead of a hang.
+// arbitrary inputs: the version read rule, TXPreValidation, TXWriteBack's slot choice, the
+// bounded wait that turns a wait nobody satisfies into an error status instead of a hang, and the
+// engine's clock advance (complete_range).
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "../../../include/csmv_tx.cuh"
+#include "../bank_kernel.cuh"
 
 using namespace csmv;
 
@@ -68,6 +70,17 @@ __global__ void bounded_wait_kernel(uint32_t* flag, uint32_t* err, uint32_t limi
   const bool ok = bounded_wait([&] { return ld_acquire_gpu(flag) != 0; }, err, ERR_WAIT_TURN,
                                limit_log2);
   if (threadIdx.x == 0) *done = ok ? 1u : 2u;
+}
+
+// Warp w completes the ranges [lo[i], hi[i]], i = w, w + warps, ..., and records the clock it then
+// sees.
+__global__ void complete_kernel(uint32_t* done, uint32_t done_mask, GlobalSync* gs,
+                                const uint32_t* lo, const uint32_t* hi, uint32_t n, uint32_t* clock) {
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / 32, nw = gridDim.x * blockDim.x / 32;
+  for (uint32_t i = w; i < n; i += nw) {
+    complete_range(done, done_mask, gs, lo[i], hi[i]);
+    if (lane_id() == 0) clock[i] = ld_acquire_gpu(&gs->clock);
+  }
 }
 
 template <class T>
@@ -149,6 +162,32 @@ int csmv_devtest_writeback(uint64_t* slots, int depth, uint32_t n_items, const u
   cudaFree(dst);
   cudaFree(dts);
   cudaFree(dv);
+  return rc;
+}
+
+// Completes n ranges of timestamps after clock0 with `warps` warps (1: in order); clock[i] = the
+// clock seen after range i, done_out = the bitmap at the end.
+int csmv_devtest_complete(uint32_t done_mask, uint32_t clock0, const uint32_t* lo,
+                          const uint32_t* hi, uint32_t n, uint32_t warps, uint32_t* clock,
+                          uint32_t* clock_end, uint32_t* done_out) {
+  GlobalSync g{}, *dg;
+  g.clock = clock0;
+  uint32_t *dd, *dl, *dh, *dc;
+  int rc = to_dev(&dd, (const uint32_t*)nullptr, (size_t)done_mask + 1) | to_dev(&dg, &g, 1) |
+           to_dev(&dl, lo, n) | to_dev(&dh, hi, n) | to_dev(&dc, (const uint32_t*)nullptr, n);
+  if (rc) return rc;
+  cudaMemset(dd, 0, ((size_t)done_mask + 1) * 4);
+  complete_kernel<<<(warps + 3) / 4, warps < 4 ? 32 * warps : 128>>>(dd, done_mask, dg, dl, dh, n, dc);
+  if (cudaMemcpy(clock, dc, (size_t)n * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+      cudaMemcpy(done_out, dd, ((size_t)done_mask + 1) * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+      cudaMemcpy(&g, dg, sizeof(g), cudaMemcpyDeviceToHost) != cudaSuccess)
+    rc = 2;
+  *clock_end = g.clock;
+  cudaFree(dd);
+  cudaFree(dg);
+  cudaFree(dl);
+  cudaFree(dh);
+  cudaFree(dc);
   return rc;
 }
 

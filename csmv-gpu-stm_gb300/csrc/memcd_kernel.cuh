@@ -422,11 +422,8 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
         else
           st_relaxed_gpu(owner_word(p.cw, target), 0u);
       }
-      __syncwarp();
-      if (lane == 0) {
-        complete_range(p.done, p.done_mask, p.gs, base + 1, base + __popc(cand));
-        stat_add(sm.stat, ST_COMMIT_UPDATE, __popc(okm));
-      }
+      complete_range(p.done, p.done_mask, p.gs, base + 1, base + __popc(cand));
+      if (lane == 0) stat_add(sm.stat, ST_COMMIT_UPDATE, __popc(okm));
       pending &= ~okm;
       uint32_t err = 0;
       if (lane == 0) err = ld_relaxed_gpu(&p.gs->error);

@@ -26,6 +26,9 @@ def dt():
     d.csmv_devtest_prevalidate.argtypes = [C.c_void_p] * 5 + [C.c_uint32, C.c_void_p]
     d.csmv_devtest_writeback.argtypes = [C.c_void_p, C.c_int, C.c_uint32, C.c_void_p, C.c_void_p, C.c_void_p]
     d.csmv_devtest_bounded_wait.argtypes = [C.c_uint32, C.c_void_p, C.c_void_p]
+    d.csmv_devtest_complete.restype = C.c_int
+    d.csmv_devtest_complete.argtypes = [C.c_uint32, C.c_uint32, C.c_void_p, C.c_void_p, C.c_uint32,
+                                        C.c_uint32, C.c_void_p, C.c_void_p, C.c_void_p]
     return d
 
 
@@ -131,3 +134,49 @@ def test_bounded_wait_returns_error_instead_of_hanging(dt):
     err, done = C.c_uint32(), C.c_uint32()
     assert dt.csmv_devtest_bounded_wait(12, C.byref(err), C.byref(done)) == 0
     assert err.value == 1 and done.value == 2
+
+
+@pytest.mark.parametrize("clock0,sizes,order", [
+    (0, [32] * 8, "forward"),              # whole words
+    (7, [1] * 70, "random"),               # single timestamps across two word boundaries
+    (31, [32, 1, 31, 2, 32, 32], "first_last"),
+    (1000, None, "random"),                # every size, word-straddling ranges
+    (2040, None, "first_last"),            # backlog of more than one 1024-timestamp step, wrapping
+    (65536 * 32 - 5, None, "random"),
+])
+def test_clock_advance_over_completed_prefix(dt, clock0, sizes, order):
+    """One warp: after each range the clock is the end of the longest complete prefix (so never
+    inside a range), and the bitmap words it passed are clear for the next lap. Many warps on
+    the same ranges at once leave the same final clock and bitmap."""
+    rng = np.random.default_rng(clock0)
+    if sizes is None:
+        sizes = rng.integers(1, 33, 100).tolist()
+    end = clock0 + np.cumsum(sizes)
+    lo = (end - sizes + 1).astype(np.uint32)
+    hi = end.astype(np.uint32)
+    perm = np.arange(len(sizes))
+    if order == "random":
+        rng.shuffle(perm)
+    elif order == "first_last":
+        perm = np.roll(perm, -1)
+    lo, hi, done_mask = lo[perm].copy(), hi[perm].copy(), 127  # ring of 4096 timestamps
+    want, got, at = [], set(), 0
+    for i in perm:
+        got.add(int(i))
+        while at in got:
+            at += 1
+        want.append(clock0 + sum(sizes[:at]))
+    last = int(end[-1])
+    for warps in (1, 64):
+        clock, done = np.zeros(len(sizes), np.uint32), np.zeros(done_mask + 1, np.uint32)
+        fin = C.c_uint32()
+        assert dt.csmv_devtest_complete(done_mask, clock0, p(lo), p(hi), len(sizes), warps, p(clock),
+                                        C.byref(fin), p(done)) == 0
+        if warps == 1:
+            np.testing.assert_array_equal(clock, np.array(want, np.uint32))
+        assert fin.value == last
+        left = np.zeros(done_mask + 1, np.uint32)  # only the last, unfinished word keeps its bits
+        first_bit = max(last + 1 & ~31, clock0 + 1)
+        for t in range(first_bit, last + 1):
+            left[(t >> 5) & done_mask] |= np.uint32(1 << (t & 31))
+        np.testing.assert_array_equal(done, left)
