@@ -445,3 +445,21 @@ def test_engine_and_serial_lane_runs_interleave_exactly():
     err = orc.check(s.op, s.off, s.addr, n_acc, np.full(n_acc, 1000, np.int32), 4, prev,
                     np.concatenate(logs), np.concatenate(outs), np.concatenate(ress), slots)
     assert err is None, err
+
+
+@pytest.mark.parametrize("n", [2, 31, 1001])
+@pytest.mark.parametrize("depth", [2, 4, 8, 16])
+def test_values_are_the_newest_versions(depth, n):
+    """The balances read back are each account's version of the largest timestamp: freshly loaded
+    accounts (one version, the rest empty) and written ones, negative balances among them."""
+    w = c1_workload(n_txn=32 * 40, n_accounts=n, up_reads=2, kind=cg.KIND_TRANSFER_ALWAYS, seed=n)
+    init = np.random.default_rng(n).integers(-2**31, 2**31, n).astype(np.int32)
+    with cg.Bank(n_accounts=n, version_depth=depth, max_txn=w.n_txn, ctas=2, client_warps=2) as bank:
+        bank.load(init)
+        np.testing.assert_array_equal(bank.values(), init)
+        bank.run(cg.generate(w))
+        v = bank.versions().reshape(n, depth)
+        ts = (v >> np.uint64(32)).astype(np.int64)
+        ts[ts == 0xFFFFFFFF] = -1
+        newest = v[np.arange(n), ts.argmax(1)]
+        np.testing.assert_array_equal(bank.values(), newest.astype(np.uint32).view(np.int32))
