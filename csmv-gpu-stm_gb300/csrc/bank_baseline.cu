@@ -194,13 +194,12 @@ __global__ void __launch_bounds__(512, 1) baseline_kernel(BankParams p) {
         if (moved) {
           SlotEditor<DEPTH> ed;
           ed.load(p.slots + (size_t)a[1] * DEPTH);
-          ed.insert(my_ts, w1);  // a transfer writes a1 last (a0 == a1 keeps the credit)
-          ed.store(p.slots + (size_t)a[1] * DEPTH);
+          // a transfer writes a1 last (a0 == a1 keeps the credit)
+          ed.install(p.slots + (size_t)a[1] * DEPTH, my_ts, w1);
           st_relaxed_gpu(&p.cw[a[1]], (unsigned long long)my_ts);
           if (a[0] != a[1]) {
             ed.load(p.slots + (size_t)a[0] * DEPTH);
-            ed.insert(my_ts, w0);
-            ed.store(p.slots + (size_t)a[0] * DEPTH);
+            ed.install(p.slots + (size_t)a[0] * DEPTH, my_ts, w0);
             st_relaxed_gpu(&p.cw[a[0]], (unsigned long long)my_ts);
           }
         }

@@ -66,6 +66,7 @@ struct alignas(128) GlobalSync {
   alignas(128) unsigned long long turn;  // ring protocol: low 32 ticket served, high 32 last ts
   alignas(128) uint32_t ticket;          // ring protocol: next ticket
   alignas(128) uint32_t clock;           // every commit with ts <= clock is written back
+  alignas(128) uint32_t advancing;       // 1 while a warp moves the clock (complete_range)
   alignas(128) uint32_t ts_next;         // stamp protocol: last timestamp handed out
   alignas(128) uint32_t round_next;      // next unclaimed round of the stream (main queue)
   alignas(128) uint32_t round_deferred;  // next unclaimed round of the deferred queue
@@ -179,6 +180,9 @@ struct GroupScratch {
   uint32_t md[32], mm[32];    // divisor and its multiply-shift magic
 };
 
+// Polls (about 0.6 us each) a group that holds locks makes for a missing one before it queues.
+constexpr uint32_t kGrpSpinPolls = 8;
+
 __host__ __device__ constexpr size_t group_scratch_offset(size_t cta_bytes) {
   return (cta_bytes + 15u) & ~size_t(15u);
 }
@@ -259,8 +263,7 @@ __device__ __forceinline__ bool transfer_writes(uint32_t op, uint32_t nr, const 
   return CSMV_OP_KIND(op) == CSMV_KIND_TRANSFER_ALWAYS || v[0] >= (int32_t)amt;
 }
 
-// Install versions (ts, value) into an item whose lock the caller holds: `n` insertions applied
-// to the item's slots in registers (victim = empty, else oldest), then stored back.
+// An item's version slots in registers, for a caller that holds its lock and installs a version.
 template <int DEPTH>
 struct SlotEditor {
   unsigned long long s[DEPTH];
@@ -268,8 +271,9 @@ struct SlotEditor {
 #pragma unroll
     for (int d = 0; d < DEPTH; d += 2) ld_relaxed_gpu_v2(item + d, s[d], s[d + 1]);
   }
-  __device__ __forceinline__ void insert(uint32_t ts, int32_t v) {
-    int vic = 0;
+  // Slot a new version replaces: empty, else the oldest (lowest index on ties).
+  __device__ __forceinline__ uint32_t victim() const {
+    uint32_t vic = 0;
     uint32_t key = version_ts(s[0]) + 1u;
 #pragma unroll
     for (int d = 1; d < DEPTH; d++) {
@@ -279,13 +283,12 @@ struct SlotEditor {
         vic = d;
       }
     }
-#pragma unroll
-    for (int d = 0; d < DEPTH; d++)
-      if (d == vic) s[d] = pack_version(ts, v);
+    return vic;
   }
-  __device__ __forceinline__ void store(unsigned long long* item) const {
-#pragma unroll
-    for (int d = 0; d < DEPTH; d++) st_relaxed_gpu(item + d, s[d]);
+  // The new version replaces the victim of the slots as loaded, in the item: one 8-byte store,
+  // not the item's DEPTH - the release that follows waits for every store.
+  __device__ __forceinline__ void install(unsigned long long* item, uint32_t ts, int32_t v) const {
+    st_relaxed_gpu(item + victim(), pack_version(ts, v));
   }
   // value of the version with timestamp ts (false when the slots do not hold it)
   __device__ __forceinline__ bool find(uint32_t ts, int32_t& v) const {
@@ -304,68 +307,99 @@ struct SlotEditor {
 // clock: completion bitmap
 // ---------------------------------------------------------------------------------------------
 
-// Mark timestamps [lo, hi] (hi - lo < 32) complete (their write-back is visible), then move the
-// clock over the longest complete prefix; warp-collective. Any warp may advance: a CAS keeps the
-// clock monotonic, and the warp that passes the end of a bitmap word clears it for the next lap.
-// A range is published atomically for the clock: of its (at most two) bitmap words the higher is
-// set first, fenced, then the lower, so a scan that sees the range's first bit and reads the next
-// word after it sees all of it - the clock never stops inside a range (a group commit's
-// intermediate versions are never installed, and no snapshot may fall between them).
+// Longest complete prefix of timestamps above c: its end. Lane l reads word l of the next 32
+// (1024 timestamps a step): one word a step, a dependent L2 round trip (about 0.28 us) per 32
+// timestamps, was what the whole engine waited for - 2^20 uncontended transactions (26 K words)
+// took 7.4 ms, and 1.4 ms with this scan. The scan runs to the first incomplete timestamp, never
+// a fixed number of words (a scan cut short could end inside a range and publish a clock no
+// snapshot may take), at most over the whole bitmap, which holds every timestamp in flight.
+// Words read together are not ordered, so a scan that stops at a word's first bit - where a
+// range's upper part may be missing - reads that word again. Warp-collective.
+static __device__ uint32_t complete_prefix(const uint32_t* done, uint32_t done_mask, uint32_t c) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  const uint32_t lane = lane_id();
+  uint32_t n = c;
+  for (uint32_t words = 0; words <= done_mask + 32u; words += 32u) {
+    const uint32_t first = (n + 1u) >> 5, bit = (n + 1u) & 31u;
+    uint32_t w = ld_acquire_gpu(&done[(first + lane) & done_mask]);
+    if (lane == 0) w |= (1u << bit) - 1u;
+    const uint32_t open = __ballot_sync(FULL, w != FULL);
+    if (open == 0u) {
+      n = ((first + 32u) << 5) - 1u;
+      continue;
+    }
+    const uint32_t k = __ffs(open) - 1u;
+    const uint32_t b = __ffs(~__shfl_sync(FULL, w, k)) - 1u;
+    n = ((first + k) << 5) + b - 1u;
+    if (b != 0u || k == 0u) break;
+  }
+  return n;
+}
+
+// Mark timestamps [lo, hi] (hi - lo < 32) complete (their write-back is visible), then see that the
+// clock moves over the longest complete prefix; warp-collective. A range is published atomically
+// for the clock: of its (at most two) bitmap words the higher is set first, fenced, then the
+// lower, so a scan that sees the range's first bit and reads the next word after it sees all of
+// it - the clock never stops inside a range (a group commit's intermediate versions are never
+// installed, and no snapshot may fall between them).
+// One warp at a time moves the clock (gs->advancing); a warp that finds another at it leaves its
+// range to that one, which looks again after it has stepped down. (Every completing warp used to
+// scan and race a CAS on the clock: with 21 ranges completed per us on an uncontended bank about
+// 50 scanned the same words at once, and completion took 13 to 38 us of a round.)
 static __device__ void complete_range(uint32_t* done, uint32_t done_mask, GlobalSync* gs, uint32_t lo,
                                uint32_t hi) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = lane_id();
   __syncwarp();
+  uint32_t busy = 0;
   if (lane == 0) {
-    __threadfence();
+    fence_acq_rel_gpu();
     const uint32_t wl = lo >> 5, wh = hi >> 5, up = FULL >> (31u - (hi & 31u)), dn = FULL << (lo & 31u);
     if (wh != wl) {
       atomicOr(&done[wh & done_mask], up);
-      __threadfence();
+      fence_acq_rel_gpu();
     }
     atomicOr(&done[wl & done_mask], wh != wl ? dn : up & dn);
-    // store-buffering pattern with the warp completing the range below ours: with SC fences on
-    // both sides at least one of us sees the other's bits, so the clock never stalls
-    __threadfence();
+    // store buffering with the warp that steps down: SC fences on both sides, so either this
+    // exchange finds the place free or that warp's last look sees these bits
+    fence_sc_gpu();
+    busy = atomicExch(&gs->advancing, 1u);
+    if (!busy) fence_acq_rel_gpu();  // what the last advancing warp wrote is read below
   }
+  busy = __shfl_sync(FULL, busy, 0);
+  if (busy) return;
   __syncwarp();
-  for (uint32_t attempt = 0; attempt < 4096; attempt++) {
-    uint32_t c = 0;
-    if (lane == 0) c = ld_acquire_gpu(&gs->clock);
-    c = __shfl_sync(FULL, c, 0);
-    uint32_t n = c;
-    // Scan to the first incomplete timestamp, never a fixed number of words: a scan cut short
-    // could end inside a range and publish a clock no snapshot may take (at most the whole
-    // bitmap, which holds every timestamp in flight). The lanes read 32 words (1024 timestamps)
-    // at once: one word a step, a dependent L2 round trip (about 0.28 us) per 32 timestamps, was
-    // what the whole engine waited for - 2^20 uncontended transactions (26 K words) took 7.4 ms,
-    // and take 1.4 ms. Words read together are not ordered, so a scan that stops at a word's
-    // first bit - where a range's upper part may be missing - reads that word again.
-    for (uint32_t words = 0; words <= done_mask + 32u; words += 32u) {
-      const uint32_t first = (n + 1u) >> 5, bit = (n + 1u) & 31u;
-      uint32_t w = ld_acquire_gpu(&done[(first + lane) & done_mask]);
-      if (lane == 0) w |= (1u << bit) - 1u;
-      const uint32_t open = __ballot_sync(FULL, w != FULL);
-      if (open == 0u) {
-        n = ((first + 32u) << 5) - 1u;
-        continue;
+  uint32_t c = ld_acquire_gpu(&gs->clock);  // only the advancing warp moves it
+  for (;;) {  // every pass moves the clock or steps down
+    const uint32_t n = complete_prefix(done, done_mask, c);
+    __syncwarp();
+    if (n != c) {
+      if (lane == 0) {
+        fence_acq_rel_gpu();
+        st_relaxed_gpu(&gs->clock, n);
       }
-      const uint32_t k = __ffs(open) - 1u;
-      const uint32_t b = __ffs(~__shfl_sync(FULL, w, k)) - 1u;
-      n = ((first + k) << 5) + b - 1u;
-      if (b != 0u || k == 0u) break;
-    }
-    if (n == c) return;  // c+1 not complete yet: its owner will advance past us
-    uint32_t won = 0;
-    if (lane == 0) {
-      __threadfence();
-      won = atomicCAS(&gs->clock, c, n) == c ? 1u : 0u;
-    }
-    if (__shfl_sync(FULL, won, 0)) {
-      // clear every word whose last timestamp this advance passed
+      // clear every word whose last timestamp this advance passed, for the next lap
       for (uint32_t wd = ((c + 1u) >> 5) + lane; wd * 32u + 31u <= n && wd <= (n >> 5); wd += 32u)
         st_relaxed_gpu(&done[wd & done_mask], 0u);
+      c = n;
+      continue;
     }
+    if (lane == 0) {
+      fence_acq_rel_gpu();
+      st_relaxed_gpu(&gs->advancing, 0u);
+      fence_sc_gpu();
+      const uint32_t t = c + 1u;  // the last look: the owner of c + 1 may have found us here
+      busy = (ld_relaxed_gpu(&done[(t >> 5) & done_mask]) >> (t & 31u)) & 1u
+                 ? atomicExch(&gs->advancing, 1u)
+                 : 1u;
+      if (!busy) {
+        fence_acq_rel_gpu();
+        c = ld_relaxed_gpu(&gs->clock);
+      }
+    }
+    busy = __shfl_sync(FULL, busy, 0);
+    if (busy) return;
+    c = __shfl_sync(FULL, c, 0);
   }
 }
 
@@ -391,25 +425,10 @@ __device__ __forceinline__ void batch_done(const BankParams& p, CtaShared<MAXR, 
 // group commit (prevalidate == 3, stamp protocol)
 // ---------------------------------------------------------------------------------------------
 
-// Lock of account x by a 64-bit CAS of its commit word from (stamp, free) to (stamp, owner):
-// the lock and, in the same atomic, a check that `stamp` (the version the caller read) is still
-// the latest. When only the stamp moved, the lock is taken at the new stamp and *stale is set
-// (the caller re-reads the value under the lock). False when another warp holds the lock.
+// A lock is taken by a 64-bit CAS of its commit word from (stamp, free) to (stamp, owner): the lock
+// and, in the same atomic, a check that `stamp` (the version the caller read) is still the latest.
 __device__ __forceinline__ unsigned long long lock_word(uint32_t stamp, uint32_t owner) {
   return ((unsigned long long)owner << 32) | stamp;
-}
-
-__device__ __forceinline__ bool group_cas_lock(unsigned long long* cw, uint32_t x, uint32_t me,
-                                               uint32_t& stamp, bool& stale) {
-  for (int r = 0; r < 8; r++) {
-    const unsigned long long exp = stamp;
-    const unsigned long long old = atomicCAS(cw + x, exp, exp | ((unsigned long long)me << 32));
-    if (old == exp) return true;
-    if ((old >> 32) != 0ull) return false;
-    stamp = (uint32_t)old;
-    stale = true;
-  }
-  return false;
 }
 
 // Lock queues. Waiters for account x queue first-come first-served on the account's ticket pair
@@ -417,7 +436,7 @@ __device__ __forceinline__ bool group_cas_lock(unsigned long long* cw, uint32_t 
 // is served (its turn), then takes the lock as soon as its holder releases it, and serves the
 // next ticket - so only the head of the queue polls the commit word, and a waiter far from the
 // account's L2 slice is not overtaken forever by nearer ones (a plain polling race hands a hot
-// lock to whoever sees the release first). A round's fast path (group_cas_lock) may still take a
+// lock to whoever sees the release first). A round's fast path (its first try) may still take a
 // free lock ahead of the queue. A waiter never leaves the queue while its run is healthy (the
 // tickets behind it would wait forever): the waits are bounded only by the device error word and
 // by 2^spin_log2 polls, after which the run fails with ERR_WAIT_TURN.
@@ -440,55 +459,19 @@ __device__ __forceinline__ void group_pass_turn(const BankParams& p, uint32_t x)
   atomicAdd(p.tk + 2u * (size_t)x + 1u, 1u);
 }
 
-// At the head of x's queue: waits for the holder's release and takes the lock, with the account's
-// version slots (ed) and latest value (v) read as it is taken. The poll that finds the lock free
-// is an acquire load, so the slots loaded after it hold the version of the stamp it saw, and a
-// CAS that succeeds at that stamp proves them current (*stale stays false).
-template <int DEPTH>
-__device__ __forceinline__ bool group_lock_at_turn(const BankParams& p, uint32_t x, uint32_t me,
-                                                   uint32_t& stamp, bool& stale,
-                                                   SlotEditor<DEPTH>& ed, int32_t& v) {
-  const uint64_t limit = 1ull << min(p.spin_log2, 22u);
-  for (uint64_t it = 0; it < limit; it++) {
-    const unsigned long long w = ld_acquire_gpu(&p.cw[x]);
-    if ((w >> 32) == 0ull) {
-      ed.load(p.slots + (size_t)x * DEPTH);
-      if (atomicCAS(&p.cw[x], w, w | ((unsigned long long)me << 32)) == w) {
-        stamp = (uint32_t)w;
-        stale = !ed.find(stamp, v);
-        return true;
-      }
-      continue;  // a fast-path CAS took it first: poll again
-    }
-    if ((it & 63u) == 63u && ld_relaxed_gpu(&p.gs->error) != 0u) break;
-    __nanosleep(32);
-  }
-  raise_error(&p.gs->error, ERR_WAIT_TURN);
-  return false;
-}
-
 // x's lock seen free as the word w (an acquire load): its slots are read and the lock taken by a
 // CAS at that stamp (false when another warp took it first).
 template <int DEPTH>
 __device__ __forceinline__ bool group_take_seen(const BankParams& p, uint32_t x, uint32_t me,
                                                 unsigned long long w, uint32_t& stamp, bool& stale,
-                                                SlotEditor<DEPTH>& ed, int32_t& v) {
+                                                uint32_t& vic, int32_t& v) {
+  SlotEditor<DEPTH> ed;
   ed.load(p.slots + (size_t)x * DEPTH);
   if (atomicCAS(&p.cw[x], w, w | ((unsigned long long)me << 32)) != w) return false;
   stamp = (uint32_t)w;
   stale = !ed.find(stamp, v);
+  vic = ed.victim();
   return true;
-}
-
-// Queue for x's lock and take it (the turn is served on, also when the wait failed).
-template <int DEPTH>
-__device__ __forceinline__ bool group_wait_lock(const BankParams& p, uint32_t x, uint32_t me,
-                                                uint32_t& stamp, bool& stale,
-                                                SlotEditor<DEPTH>& ed, int32_t& v) {
-  if (!group_take_turn(p, x)) return false;
-  const bool got = group_lock_at_turn<DEPTH>(p, x, me, stamp, stale, ed, v);
-  group_pass_turn(p, x);
-  return got;
 }
 
 // One attempt of a transfer round as a commit group, warp-collective. Every active lane's
@@ -554,7 +537,7 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   //    commits. Waits follow the order turns < cold locks < hot locks, a group holds at most
   //    one turn, and a hot lock is held only by a group that holds every smaller lock it needs
   //    or is committing: no cycle of waits. A leader keeps the account's version slots from its
-  //    read: the write-back edits them in registers.
+  //    read: the write-back picks the victim from them.
   const uint32_t c0 = (lead0 && p.lock_last != nullptr) ? p.lock_last[a[0]] : 0u;
   const uint32_t c1 = (lead1 && p.lock_last != nullptr) ? p.lock_last[a[1]] : 0u;
   // order key: (tier | class, account); tier bit 31 set for hot accounts
@@ -570,20 +553,57 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   };
   uint32_t st0 = 0, st1 = 0;
   int32_t bv0 = 0, bv1 = 0;
-  SlotEditor<DEPTH> ed0, ed1;
+  // of a led account's slots only the latest value and the next victim are kept: two words
+  // instead of 2 x DEPTH, which leaves registers for the foreign reads to run side by side
+  uint32_t vic0 = 0, vic1 = 0;
   bool stale0 = false, stale1 = false, h0 = false, h1 = false;
-  if (lead0) {
-    st0 = (uint32_t)ld_acquire_gpu(&p.cw[a[0]]);
-    ed0.load(p.slots + (size_t)a[0] * DEPTH);
-  }
-  if (lead1) {
-    st1 = (uint32_t)ld_acquire_gpu(&p.cw[a[1]]);
-    ed1.load(p.slots + (size_t)a[1] * DEPTH);
-  }
-  if (lead0) stale0 = !ed0.find(st0, bv0);
-  if (lead1) stale1 = !ed1.find(st1, bv1);
-  if (lead0) h0 = group_cas_lock(p.cw, a[0], me, st0, stale0);
-  if (lead1) h1 = group_cas_lock(p.cw, a[1], me, st1, stale1);
+  auto look = [&](uint32_t x, uint32_t& st, bool& stale, int32_t& v, uint32_t& vic) {
+    SlotEditor<DEPTH> ed;
+    st = (uint32_t)ld_acquire_gpu(&p.cw[x]);
+    ed.load(p.slots + (size_t)x * DEPTH);
+    stale = !ed.find(st, v);
+    vic = ed.victim();
+  };
+  if (lead0) look(a[0], st0, stale0, bv0, vic0);
+  if (lead1) look(a[1], st1, stale1, bv1, vic1);
+  // Takes the locks t0 / t1 of this lane's two accounts, whose words were seen free as w0 / w1,
+  // both CASes in flight together; slots read at an older stamp are read again beside the CAS,
+  // which proves them current when it succeeds. The words found by the CASes are left in w0, w1.
+  // (warp-collective)
+  auto take = [&](bool t0, unsigned long long& w0, bool t1, unsigned long long& w1) {
+    const bool n0 = t0 && (uint32_t)w0 != st0, n1 = t1 && (uint32_t)w1 != st1;
+    if (__any_sync(FULL, n0 || n1)) {
+      fence_acq_rel_gpu();  // the versions of the stamps seen are visible before they are read
+    }
+    SlotEditor<DEPTH> ed0{}, ed1{};  // (set on every path: left open, the arrays spilled)
+    if (n0) ed0.load(p.slots + (size_t)a[0] * DEPTH);
+    if (n1) ed1.load(p.slots + (size_t)a[1] * DEPTH);
+    unsigned long long o0 = ~0ull, o1 = ~0ull;
+    if (t0) o0 = atomicCAS(&p.cw[a[0]], w0, w0 | ((unsigned long long)me << 32));
+    if (t1) o1 = atomicCAS(&p.cw[a[1]], w1, w1 | ((unsigned long long)me << 32));
+    if (n0) {
+      st0 = (uint32_t)w0;
+      stale0 = !ed0.find(st0, bv0);
+      vic0 = ed0.victim();
+    }
+    if (n1) {
+      st1 = (uint32_t)w1;
+      stale1 = !ed1.find(st1, bv1);
+      vic1 = ed1.victim();
+    }
+    h0 |= t0 && o0 == w0;
+    h1 |= t1 && o1 == w1;
+    w0 = o0;
+    w1 = o1;
+  };
+  // ... and once more the ones that were free but written since they were read
+  auto take_twice = [&](bool t0, bool t1) {
+    unsigned long long w0 = st0, w1 = st1;
+    take(t0, w0, t1, w1);
+    const bool r0 = t0 && !h0 && (w0 >> 32) == 0ull, r1 = t1 && !h1 && (w1 >> 32) == 0ull;
+    if (__any_sync(FULL, r0 || r1)) take(r0, w0, r1, w1);
+  };
+  take_twice(lead0, lead1);
   if (lead0 && !h0) gx.busy[s0] = 1u;
   if (lead1 && !h1) gx.busy[s1] = 1u;
   __syncwarp();
@@ -621,16 +641,15 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
       // queued one is still held
       const bool o0 = lead0 && !h0 && turn != 0, o1 = lead1 && !h1 && turn != 1;
       unsigned long long wq = ~0ull, w0 = ~0ull, w1 = ~0ull;
-      if (turn == 0) wq = ld_acquire_gpu(&p.cw[a[0]]);
-      if (turn == 1) wq = ld_acquire_gpu(&p.cw[a[1]]);
       if (o0) w0 = ld_relaxed_gpu(&p.cw[a[0]]);
       if (o1) w1 = ld_relaxed_gpu(&p.cw[a[1]]);
+      if (turn == 0) wq = ld_acquire_gpu(&p.cw[a[0]]);  // last: nothing waits behind it
+      if (turn == 1) wq = ld_acquire_gpu(&p.cw[a[1]]);
       if (__any_sync(FULL, turn >= 0 && (wq >> 32) == 0ull)) {
-        if (turn == 0 && (wq >> 32) == 0ull) h0 = group_take_seen<DEPTH>(p, a[0], me, wq, st0, stale0, ed0, bv0);
-        if (turn == 1 && (wq >> 32) == 0ull) h1 = group_take_seen<DEPTH>(p, a[1], me, wq, st1, stale1, ed1, bv1);
+        if (turn == 0 && (wq >> 32) == 0ull) h0 = group_take_seen<DEPTH>(p, a[0], me, wq, st0, stale0, vic0, bv0);
+        if (turn == 1 && (wq >> 32) == 0ull) h1 = group_take_seen<DEPTH>(p, a[1], me, wq, st1, stale1, vic1, bv1);
       } else {
-        if (o0 && (w0 >> 32) == 0ull) h0 = group_cas_lock(p.cw, a[0], me, st0, stale0);
-        if (o1 && (w1 >> 32) == 0ull) h1 = group_cas_lock(p.cw, a[1], me, st1, stale1);
+        take(o0 && (w0 >> 32) == 0ull, w0, o1 && (w1 >> 32) == 0ull, w1);
       }
       if (__any_sync(FULL, (turn == 0 && h0) || (turn == 1 && h1))) {
         all = true;
@@ -640,10 +659,10 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
                              __any_sync(FULL, (lead0 && !h0 && turn != 0) || (lead1 && !h1 && turn != 1));
              g++) {
           __nanosleep(32);
-          if (lead0 && !h0 && turn != 0 && (ld_relaxed_gpu(&p.cw[a[0]]) >> 32) == 0ull)
-            h0 = group_cas_lock(p.cw, a[0], me, st0, stale0);
-          if (lead1 && !h1 && turn != 1 && (ld_relaxed_gpu(&p.cw[a[1]]) >> 32) == 0ull)
-            h1 = group_cas_lock(p.cw, a[1], me, st1, stale1);
+          unsigned long long x0 = ~0ull, x1 = ~0ull;
+          if (lead0 && !h0 && turn != 0) x0 = ld_relaxed_gpu(&p.cw[a[0]]);
+          if (lead1 && !h1 && turn != 1) x1 = ld_relaxed_gpu(&p.cw[a[1]]);
+          take((x0 >> 32) == 0ull, x0, (x1 >> 32) == 0ull, x1);
         }
         break;
       }
@@ -661,24 +680,59 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
         all = true;
         break;
       }
-      if (h0 && above(kh0, a[0], fh, fl)) {  // hold nothing above the lock being waited for
-        st_relaxed_gpu(&p.cw[a[0]], (unsigned long long)st0);
-        h0 = false;
+      // The warp waits together. The lane of the smallest missing lock queues for it (a hot lock
+      // is polled: its queue's turn is this group's or another's) and at the head polls it; the
+      // other lanes look at their missing words in the same round of loads, and when the awaited
+      // lock is seen free every lock seen free is taken at once, so a hot lock is not held
+      // while the others are collected (on the Zipf(0.99) bank in stream order that took 3.2 us
+      // of a 11.8 us hold). A group that already holds locks first polls a few times without
+      // queueing: what it misses is mostly being released by a group that commits now.
+      const bool q0 = lead0 && !h0 && kh0 == fh && a[0] == fl;
+      const bool q1 = !q0 && lead1 && !h1 && kh1 == fh && a[1] == fl;
+      const bool tickets = (q0 && !c0) || (q1 && !c1);
+      const uint32_t spin = __any_sync(FULL, h0 || h1) ? kGrpSpinPolls : 0u;
+      const uint64_t limit = 1ull << min(p.spin_log2, 22u);
+      bool r = true, queued = false, got = false;
+      for (uint64_t n = 0; n < limit; n++) {
+        // hold nothing above the lock being waited for
+        if (h0 && above(kh0, a[0], fh, fl)) {
+          st_relaxed_gpu(&p.cw[a[0]], (unsigned long long)st0);
+          h0 = false;
+        }
+        if (h1 && above(kh1, a[1], fh, fl)) {
+          st_relaxed_gpu(&p.cw[a[1]], (unsigned long long)st1);
+          h1 = false;
+        }
+        if (n == spin) {
+          if (tickets) queued = r = group_take_turn(p, fl);
+          if (__any_sync(FULL, !r)) break;
+        }
+        const bool t0 = lead0 && !h0, t1 = lead1 && !h1;
+        unsigned long long w0 = ~0ull, w1 = ~0ull;
+        // (the awaited word first: its holder releases the others with it)
+        if (q0) w0 = ld_relaxed_gpu(&p.cw[a[0]]);
+        if (q1) w1 = ld_relaxed_gpu(&p.cw[a[1]]);
+        if (t0 && !q0) w0 = ld_relaxed_gpu(&p.cw[a[0]]);
+        if (t1 && !q1) w1 = ld_relaxed_gpu(&p.cw[a[1]]);
+        if (__any_sync(FULL, (q0 && (w0 >> 32) == 0ull) || (q1 && (w1 >> 32) == 0ull))) {
+          const bool f0 = t0 && (w0 >> 32) == 0ull, f1 = t1 && (w1 >> 32) == 0ull;
+          take(f0, w0, f1, w1);
+          got = __any_sync(FULL, (q0 && h0) || (q1 && h1));
+          if (got) {  // once more the ones that were written since they were read
+            const bool r0 = f0 && !h0 && (w0 >> 32) == 0ull, r1 = f1 && !h1 && (w1 >> 32) == 0ull;
+            if (__any_sync(FULL, r0 || r1)) take(r0, w0, r1, w1);
+            break;
+          }
+          continue;  // a fast-path CAS took it first: poll again
+        }
+        if ((n & 63u) == 63u && __any_sync(FULL, lane == 0 && ld_relaxed_gpu(&p.gs->error) != 0u)) break;
+        __nanosleep(32);
       }
-      if (h1 && above(kh1, a[1], fh, fl)) {
-        st_relaxed_gpu(&p.cw[a[1]], (unsigned long long)st1);
-        h1 = false;
+      if (queued) group_pass_turn(p, fl);
+      if (!got) {
+        if ((q0 || q1) && r) raise_error(&p.gs->error, ERR_WAIT_TURN);
+        break;
       }
-      bool r = true;  // a hot lock is polled (its queue's turn is this group's or another's)
-      if (lead0 && !h0 && kh0 == fh && a[0] == fl)
-        r = h0 = c0 ? group_lock_at_turn<DEPTH>(p, a[0], me, st0, stale0, ed0, bv0)
-                    : group_wait_lock<DEPTH>(p, a[0], me, st0, stale0, ed0, bv0);
-      else if (lead1 && !h1 && kh1 == fh && a[1] == fl)
-        r = h1 = c1 ? group_lock_at_turn<DEPTH>(p, a[1], me, st1, stale1, ed1, bv1)
-                    : group_wait_lock<DEPTH>(p, a[1], me, st1, stale1, ed1, bv1);
-      if (__any_sync(FULL, !r)) break;
-      if (lead0 && !h0 && above(kh0, a[0], fh, fl)) h0 = group_cas_lock(p.cw, a[0], me, st0, stale0);
-      if (lead1 && !h1 && above(kh1, a[1], fh, fl)) h1 = group_cas_lock(p.cw, a[1], me, st1, stale1);
     }
   }
   if (turn >= 0) group_pass_turn(p, turn == 0 ? a[0] : a[1]);  // the next in line starts now
@@ -711,12 +765,16 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
     fence_acq_rel_gpu();  // the previous holders' versions are visible before they are read
     bool lost = false;
     if (own0 && stale0) {
-      ed0.load(p.slots + (size_t)a[0] * DEPTH);
-      lost |= !ed0.find(st0, bv0);
+      SlotEditor<DEPTH> ed;
+      ed.load(p.slots + (size_t)a[0] * DEPTH);
+      lost |= !ed.find(st0, bv0);
+      vic0 = ed.victim();
     }
     if (own1 && stale1) {
-      ed1.load(p.slots + (size_t)a[1] * DEPTH);
-      lost |= !ed1.find(st1, bv1);
+      SlotEditor<DEPTH> ed;
+      ed.load(p.slots + (size_t)a[1] * DEPTH);
+      lost |= !ed.find(st1, bv1);
+      vic1 = ed.victim();
     }
     if (lost) raise_error(&p.gs->error, ERR_DATA);  // the latest version must be present
   }
@@ -741,106 +799,181 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   uint32_t fst[MAXR];
   bool fok = true;
 #pragma unroll
-  for (int k = 0; k < MAXR; k++) {
+  for (int k = 0; k < 2; k++) {  // (its two accounts are in the table)
     fv[k] = 0;
     fst[k] = 0u;
-    if (in && k < (int)nr && rsl[k] < 0) fok &= read_latest<DEPTH>(vs, p.cw, a[k], fst[k], fv[k]);
   }
-  bool ok_wait = true;
-  if (lane == 0)  // the hottest lock is held: spin on the reply before sleeping between polls
-    ok_wait = bounded_wait_fast([&] { return mail_acquire<CLUSTER>(&ms.rep) == seq; },
-                                &p.gs->error, ERR_WAIT_REPLY, p.spin_log2);
-  ok_wait = __shfl_sync(FULL, ok_wait, 0);
-  if (!ok_wait) {
-    failed = true;
-    return 0u;
-  }
-  (void)mail_acquire<CLUSTER>(&ms.rep);
-  const uint32_t base = ms.base, n_ts = __popc(inc);
-  const uint32_t my_ts = base + 1u + __popc(inc & lanemask_lt());
-  fence_acq_rel_gpu();
-
-  // 5. the group's first timestamp in its locks, then validation of the foreign reads: the stamp
-  //    read must still be the latest, and a lock of a holder ordered before us (or whose
-  //    timestamps are being drawn) must be resolved first. Waits point only to earlier
-  //    timestamps or to holders already drawing: no cycles.
-  if (own0) st_relaxed_gpu(&p.cw[a[0]], lock_word(st0, kPendingFlag | (base + 1u)));
-  if (own1) st_relaxed_gpu(&p.cw[a[1]], lock_word(st1, kPendingFlag | (base + 1u)));
-  bool valid = in && fok;
-  if (valid) {
-    const uint32_t wait_polls = p.read_wait ? p.read_wait : 4096u;
-    unsigned long long word[MAXR];
 #pragma unroll
-    for (int k = 0; k < MAXR; k++)
-      word[k] = (k < (int)nr && rsl[k] < 0) ? ld_relaxed_gpu(&p.cw[a[k]]) : 0ull;
-#pragma unroll
-    for (int k = 0; k < MAXR; k++) {
-      if (k >= (int)nr || rsl[k] >= 0 || !valid) continue;
-      unsigned long long wd = word[k];
-      bool settled = false;  // a lane that gives up leaves a hole and is retried
-      for (uint32_t it = 0; it < wait_polls; it++) {
-        const uint32_t own = (uint32_t)(wd >> 32);
-        bool clear;
-        if (own == 0u)
-          clear = true;
-        else if (own & kPendingFlag)
-          clear = (own & ~kPendingFlag) >= my_ts;  // its group is ordered after ours
-        else
-          clear = !(own & kReadyFlag);  // still acquiring: its timestamps follow ours
-        if (clear) {
-          settled = true;
-          break;
-        }
-        __nanosleep(32);
-        wd = ld_relaxed_gpu(&p.cw[a[k]]);
-      }
-      // the reads were issued while the timestamps were being drawn, so a version read may even
-      // be newer than ours (a group ordered after us that committed meanwhile): it must be below
-      if (settled && ((uint32_t)wd != fst[k] || fst[k] >= my_ts)) {
-        // a version below our timestamp was committed since the read, and no holder ordered
-        // before us remains: that version is the latest as of our timestamp, so it is read
-        // again (the chain below has not used the value yet) instead of aborting. A version at
-        // or above our timestamp (a group ordered after us that already committed) is not.
-        uint32_t s2 = 0u;
-        int32_t v2 = 0;
-        if ((uint32_t)wd < my_ts && read_latest<DEPTH>(vs, p.cw, a[k], s2, v2) &&
-            s2 == (uint32_t)wd) {
-          fst[k] = s2;
-          fv[k] = v2;
-        } else {
-          settled = false;
-        }
-      }
-      valid = settled;
-    }
+  for (int k = 2; k < MAXR; k += 2) {  // two reads' loads in flight together
+    const bool f0 = in && k < (int)nr && rsl[k] < 0, f1 = in && k + 1 < (int)nr && rsl[k + 1] < 0;
+    SlotEditor<DEPTH> e0{}, e1{};
+    unsigned long long w0 = 0ull, w1 = 0ull;
+    if (f0) w0 = ld_relaxed_gpu(&p.cw[a[k]]);
+    if (f1) w1 = ld_relaxed_gpu(&p.cw[a[k + 1]]);
+    if (f0) e0.load(p.slots + (size_t)a[k] * DEPTH);
+    if (f1) e1.load(p.slots + (size_t)a[k + 1] * DEPTH);
+    fst[k] = (uint32_t)w0;
+    fst[k + 1] = (uint32_t)w1;
+    fv[k] = fv[k + 1] = 0;
+    // the stamp's version not visible yet (word and slots came together): the word again, then
+    // the slots after it
+    if (f0 && !e0.find(fst[k], fv[k])) fok &= read_latest<DEPTH>(vs, p.cw, a[k], fst[k], fv[k]);
+    if (f1 && !e1.find(fst[k + 1], fv[k + 1]))
+      fok &= read_latest<DEPTH>(vs, p.cw, a[k + 1], fst[k + 1], fv[k + 1]);
   }
-  const uint32_t fin = __ballot_sync(FULL, valid);
-
-  // 6. the chain, in lane order through the locked accounts. Every lane first computes its
+  // 5. the chain, in lane order through the locked accounts. Every lane first computes its
   //    transfer from the values read under the locks; that result is final for a lane no lower
   //    lane writes any of its accounts to (every writer of an account also reads it, so two
-  //    writers of one account are always dependent). When some lanes depend on lower ones, each
-  //    stages what its transfer needs (table slots, the part of its amount sum read outside the
-  //    table, its divisor) and lane 0 runs every lane from the first dependent one on, in order,
-  //    over the table's values in shared memory (a transfer writes a1 last; an independent
-  //    lane's inputs are unchanged, so it computes its result again).
-  uint32_t dep = 0u;
+  //    writers of one account are always dependent).
+  //    When no lane's amount depends on a lower lane (the transfers read only their two
+  //    accounts, or move fixed amounts), the chain is a sum: each lane adds up the amounts the
+  //    lower lanes move over its two accounts, assuming all of them move theirs. If then every
+  //    lane's funds suffice, the assumption holds (by induction in lane order) and the values
+  //    are the chain's; otherwise the walk below runs. That is 31 independent steps of one
+  //    shuffle where the walk takes up to 31 dependent ones through shared memory: on the
+  //    Zipf(0.99) bank 1.0 us of a hold instead of 3.5 us.
+  //    A first pass runs while the server draws the timestamps, for the lanes that took part;
+  //    it stands unless validation drops a lane or reads a value again.
+  const bool took = in && fok;
+  bool valid = took, changed = false;
+  uint32_t fin = __ballot_sync(FULL, took), depm = 0u, hw = 0u, base = 0u, n_ts = 0u, my_ts = 0u;
+  for (int pass = 0;; pass++) {
+    uint32_t dep = 0u;
 #pragma unroll
-  for (int k = 0; k < MAXR; k++)
-    if (valid && k < (int)nr && rsl[k] >= 0) dep |= gx.wmask[rsl[k]];
-  dep &= fin & lanemask_lt();
-  bool has_w = false;
-  if (valid) {
-    int32_t v[MAXR];
+    for (int k = 0; k < MAXR; k++)
+      if (valid && k < (int)nr && rsl[k] >= 0) dep |= gx.wmask[rsl[k]];
+    dep &= fin & lanemask_lt();
+    bool has_w = false;
+    if (valid) {
+      int32_t v[MAXR];
 #pragma unroll
-    for (int k = 0; k < MAXR; k++) v[k] = (k >= (int)nr) ? 0 : rsl[k] < 0 ? fv[k] : gx.base[rsl[k]];
-    int32_t w0 = 0, w1 = 0;
-    has_w = transfer_writes<MAXR>(op, nr, v, w0, w1);
-    gx.out0[lane] = w0;
-    gx.out1[lane] = w1;
+      for (int k = 0; k < MAXR; k++) v[k] = (k >= (int)nr) ? 0 : rsl[k] < 0 ? fv[k] : gx.base[rsl[k]];
+      int32_t w0 = 0, w1 = 0;
+      has_w = transfer_writes<MAXR>(op, nr, v, w0, w1);
+      gx.out0[lane] = w0;
+      gx.out1[lane] = w1;
+    }
+    depm = __ballot_sync(FULL, dep != 0u);
+    hw = __ballot_sync(FULL, has_w);
+    if (depm) {
+      bool adep = false;  // an amount that a lower lane's write changes
+      if (valid && CSMV_OP_AMOD(op) != 1u) {
+#pragma unroll
+        for (int k = 2; k < MAXR; k++)
+          if (k < (int)nr && rsl[k] >= 0) adep |= (gx.wmask[rsl[k]] & fin & lanemask_lt()) != 0u;
+      }
+      uint32_t amt = 0u;
+      if (valid) amt = (uint32_t)gx.base[s0] - (uint32_t)gx.out0[lane];
+      if (!__any_sync(FULL, adep || amt > 0xFFFFu)) {  // (amounts above 16 bits: no divisor)
+        const uint32_t pk = ((uint32_t)s0 & 0xFFu) | (((uint32_t)s1 & 0xFFu) << 8) | (amt << 16);
+        uint32_t d0 = 0u, d1 = 0u;
+        const uint32_t srcs = __reduce_or_sync(FULL, dep);
+        for (uint32_t m = srcs; m; m &= m - 1u) {
+          const uint32_t j = __ffs(m) - 1u, q = __shfl_sync(FULL, pk, j);
+          const uint32_t x0 = q & 0xFFu, x1 = (q >> 8) & 0xFFu, am = j < lane ? q >> 16 : 0u;
+          d0 += x1 == (uint32_t)s0 ? am : x0 == (uint32_t)s0 ? 0u - am : 0u;
+          d1 += x1 == (uint32_t)s1 ? am : x0 == (uint32_t)s1 ? 0u - am : 0u;
+        }
+        uint32_t v0 = 0u, v1 = 0u;
+        bool moved = true;
+        if (valid) {
+          v0 = (uint32_t)gx.base[s0] + d0;
+          v1 = (uint32_t)gx.base[s1] + d1;
+          moved = CSMV_OP_KIND(op) == CSMV_KIND_TRANSFER_ALWAYS || (int32_t)v0 >= (int32_t)amt;
+        }
+        if (__all_sync(FULL, moved)) {
+          if (valid) {
+            gx.out0[lane] = (int32_t)(v0 - amt);
+            gx.out1[lane] = (int32_t)(v1 + amt);
+          }
+          hw = fin;
+          depm = 0u;
+          __syncwarp();
+        }
+      }
+    }
+    if (pass) break;
+
+    // 6. the group's timestamps, the first of them in its locks, then validation of the foreign
+    //    reads: the stamp read must still be the latest, and a lock of a holder ordered before
+    //    us (or whose timestamps are being drawn) must be resolved first. Waits point only to
+    //    earlier timestamps or to holders already drawing: no cycles.
+    bool ok_wait = true;
+    if (lane == 0)  // the hottest lock is held: spin on the reply before sleeping between polls
+      ok_wait = bounded_wait_fast([&] { return mail_acquire<CLUSTER>(&ms.rep) == seq; },
+                                  &p.gs->error, ERR_WAIT_REPLY, p.spin_log2);
+    ok_wait = __shfl_sync(FULL, ok_wait, 0);
+    if (!ok_wait) {
+      failed = true;
+      return 0u;
+    }
+    (void)mail_acquire<CLUSTER>(&ms.rep);
+    base = ms.base;
+    n_ts = __popc(inc);
+    my_ts = base + 1u + __popc(inc & lanemask_lt());
+    // (every lane acquired the reply: what the server's draw acquired is ordered before the
+    // validation below, with no fence of this warp's own)
+    if (own0) st_relaxed_gpu(&p.cw[a[0]], lock_word(st0, kPendingFlag | (base + 1u)));
+    if (own1) st_relaxed_gpu(&p.cw[a[1]], lock_word(st1, kPendingFlag | (base + 1u)));
+    if (valid) {
+      const uint32_t wait_polls = p.read_wait ? p.read_wait : 4096u;
+      unsigned long long word[MAXR];
+#pragma unroll
+      for (int k = 0; k < MAXR; k++)
+        word[k] = (k < (int)nr && rsl[k] < 0) ? ld_relaxed_gpu(&p.cw[a[k]]) : 0ull;
+#pragma unroll
+      for (int k = 0; k < MAXR; k++) {
+        if (k >= (int)nr || rsl[k] >= 0 || !valid) continue;
+        unsigned long long wd = word[k];
+        bool settled = false;  // a lane that gives up leaves a hole and is retried
+        for (uint32_t it = 0; it < wait_polls; it++) {
+          const uint32_t own = (uint32_t)(wd >> 32);
+          bool clear;
+          if (own == 0u)
+            clear = true;
+          else if (own & kPendingFlag)
+            clear = (own & ~kPendingFlag) >= my_ts;  // its group is ordered after ours
+          else
+            clear = !(own & kReadyFlag);  // still acquiring: its timestamps follow ours
+          if (clear) {
+            settled = true;
+            break;
+          }
+          __nanosleep(32);
+          wd = ld_relaxed_gpu(&p.cw[a[k]]);
+        }
+        // the reads were issued while the timestamps were being drawn, so a version read may even
+        // be newer than ours (a group ordered after us that committed meanwhile): it must be below
+        if (settled && ((uint32_t)wd != fst[k] || fst[k] >= my_ts)) {
+          // a version below our timestamp was committed since the read, and no holder ordered
+          // before us remains: that version is the latest as of our timestamp, so it is read
+          // again (the chain below has not used the value yet) instead of aborting. A version at
+          // or above our timestamp (a group ordered after us that already committed) is not.
+          uint32_t s2 = 0u;
+          int32_t v2 = 0;
+          if ((uint32_t)wd < my_ts && read_latest<DEPTH>(vs, p.cw, a[k], s2, v2) &&
+              s2 == (uint32_t)wd) {
+            changed |= fv[k] != v2 && CSMV_OP_AMOD(op) != 1u;  // (an amount of amod 1 is fixed)
+            fst[k] = s2;
+            fv[k] = v2;
+          } else {
+            settled = false;
+          }
+        }
+        valid = settled;
+      }
+    }
+    const uint32_t took_m = fin;
+    fin = __ballot_sync(FULL, valid);
+    if (fin == took_m && !__any_sync(FULL, changed)) break;
   }
-  const uint32_t depm = __ballot_sync(FULL, dep != 0u);
-  uint32_t hw = __ballot_sync(FULL, has_w);
+  __syncwarp();  // every lane's outputs
+
+  // 7. the walk, when the sum does not apply: every lane stages what its transfer needs (table
+  //    slots, the part of its amount sum read outside the table, its divisor) and lane 0 runs
+  //    every lane from the first dependent one on, in order, over the table's values in shared
+  //    memory (a transfer writes a1 last; an independent lane's inputs are unchanged, so it
+  //    computes its result again).
   if (depm) {
     if (valid) {
       uint32_t facc = CSMV_OP_AMT0(op) - 1u, ntr = 0u;
@@ -932,28 +1065,27 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
     __syncwarp();
   }
 
-  // 7. one version per locked account (its last writer's), then the stamp (released: the
+  // 8. one version per locked account (its last writer's), then the stamp (released: the
   //    version is visible first) and the unlock
-  auto install = [&](int s, uint32_t x, SlotEditor<DEPTH>& ed) -> uint32_t {
+  auto install = [&](int s, uint32_t x, uint32_t vic) -> uint32_t {
     const uint32_t wr = gx.wmask[s] & hw;
     if (!wr) return 0u;
     const uint32_t j = 31u - __clz(wr);
     const int32_t val = gx.wa1[j] == x ? gx.out1[j] : gx.out0[j];
     const uint32_t ts = base + 1u + __popc(inc & ((1u << j) - 1u));
-    ed.insert(ts, val);
-    ed.store(p.slots + (size_t)x * DEPTH);
+    st_relaxed_gpu(p.slots + (size_t)x * DEPTH + vic, pack_version(ts, val));
     return ts;
   };
   uint32_t pub0 = 0u, pub1 = 0u;
-  if (own0) pub0 = install(s0, a[0], ed0);
-  if (own1) pub1 = install(s1, a[1], ed1);
+  if (own0) pub0 = install(s0, a[0], vic0);
+  if (own1) pub1 = install(s1, a[1], vic1);
   // one fence releases both words (a fence then relaxed stores is a release): two release
   // stores in a row would wait for the first to land before the second
   if (own0 || own1) fence_acq_rel_gpu();
   if (own0) st_relaxed_gpu(&p.cw[a[0]], (unsigned long long)(pub0 ? pub0 : st0));
   if (own1) st_relaxed_gpu(&p.cw[a[1]], (unsigned long long)(pub1 ? pub1 : st1));
 
-  // 8. log, outcomes, the group's end, completion
+  // 9. log, outcomes, the group's end, completion
   if (p.log && in) {
     const uint32_t li = my_ts - 1u - p.log_base;
     if (li < p.log_cap)
@@ -1359,10 +1491,7 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
                 last = ti;
               }
             }
-            if (lead && last) {
-              ed.insert(last, lv);
-              ed.store(item);
-            }
+            if (lead && last) ed.install(item, last, lv);
             __threadfence();
             if (lead) {
               if (last)
@@ -1679,11 +1808,15 @@ __device__ void server_warp_stamp(uint32_t nc, uint32_t batch, GlobalSync* gs, S
     }
     const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
     uint32_t t0 = 0;
-    if (lane == 0) {  // fences on both sides order the draw after the observed locks and
-      __threadfence();  // before the validations that follow it
-      t0 = atomicAdd(&gs->ts_next, total);
-      __threadfence();
+    // The draws' order on the cursor decides: release before the draw (the clients' lock marks)
+    // and acquire after it (their validations), so whoever draws later sees the marks of
+    // whoever drew earlier. No store-buffering pattern here, hence no SC fence.
+    __syncwarp();
+    if (lane == 0) {
+      fence_acq_rel_gpu();
+      t0 = atom_add_acquire_gpu(&gs->ts_next, total);
     }
+    __syncwarp();
     t0 = __shfl_sync(0xFFFFFFFFu, t0, 0);
     if (mine) {
       sm.mail[lane].base = t0 + incl - cnt;

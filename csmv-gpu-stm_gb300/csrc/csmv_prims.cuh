@@ -50,6 +50,11 @@ __device__ __forceinline__ unsigned long long ld_relaxed_gpu(const unsigned long
 __device__ __forceinline__ void st_relaxed_gpu(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ uint32_t atom_add_acquire_gpu(uint32_t* p, uint32_t v) {
+  uint32_t r;
+  asm volatile("atom.add.acquire.gpu.global.u32 %0, [%1], %2;" : "=r"(r) : "l"(p), "r"(v) : "memory");
+  return r;
+}
 // two 8-byte version slots in one 16-byte access; each element is single-copy atomic
 __device__ __forceinline__ void ld_relaxed_gpu_v2(const unsigned long long* p,
                                                   unsigned long long& a,
@@ -62,7 +67,8 @@ __device__ __forceinline__ void ld_relaxed_gpu_v2(const unsigned long long* p,
 __device__ __forceinline__ void fence_acq_rel_gpu() {
   asm volatile("fence.acq_rel.gpu;" ::: "memory");
 }
-
+// only where a store must not pass a later load (store buffering); costs more than acq_rel
+__device__ __forceinline__ void fence_sc_gpu() { asm volatile("fence.sc.gpu;" ::: "memory"); }
 
 // Global words shared only by the threads of one CTA (one SM): CTA scope lets the SM's L1 serve
 // them. Each 8-byte access is single-copy atomic.
