@@ -314,24 +314,30 @@ struct SlotEditor {
 // a fixed number of words (a scan cut short could end inside a range and publish a clock no
 // snapshot may take), at most over the whole bitmap, which holds every timestamp in flight.
 // Words read together are not ordered, so a scan that stops at a word's first bit - where a
-// range's upper part may be missing - reads that word again. Warp-collective.
-static __device__ uint32_t complete_prefix(const uint32_t* done, uint32_t done_mask, uint32_t c) {
+// range's upper part may be missing - reads that word again. w: the lanes' words from word
+// first on, read already. Warp-collective; the caller fences before it publishes the end.
+static __device__ uint32_t complete_prefix(const uint32_t* done, uint32_t done_mask, uint32_t c,
+                                           uint32_t first, uint32_t w) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = lane_id();
   uint32_t n = c;
+  bool have = first == (c + 1u) >> 5;
   for (uint32_t words = 0; words <= done_mask + 32u; words += 32u) {
-    const uint32_t first = (n + 1u) >> 5, bit = (n + 1u) & 31u;
-    uint32_t w = ld_acquire_gpu(&done[(first + lane) & done_mask]);
-    if (lane == 0) w |= (1u << bit) - 1u;
+    first = (n + 1u) >> 5;
+    if (!have) w = ld_relaxed_gpu(&done[(first + lane) & done_mask]);
+    have = false;
+    if (lane == 0) w |= (1u << ((n + 1u) & 31u)) - 1u;
     const uint32_t open = __ballot_sync(FULL, w != FULL);
     if (open == 0u) {
       n = ((first + 32u) << 5) - 1u;
-      continue;
+    } else {
+      const uint32_t k = __ffs(open) - 1u;
+      const uint32_t b = __ffs(~__shfl_sync(FULL, w, k)) - 1u;
+      n = ((first + k) << 5) + b - 1u;
+      if (b != 0u || k == 0u) break;
     }
-    const uint32_t k = __ffs(open) - 1u;
-    const uint32_t b = __ffs(~__shfl_sync(FULL, w, k)) - 1u;
-    n = ((first + k) << 5) + b - 1u;
-    if (b != 0u || k == 0u) break;
+    fence_acq_rel_gpu();  // the words of the next step are read after these
+    __syncwarp();
   }
   return n;
 }
@@ -345,7 +351,7 @@ static __device__ uint32_t complete_prefix(const uint32_t* done, uint32_t done_m
 // One warp at a time moves the clock (gs->advancing); a warp that finds another at it leaves its
 // range to that one, which looks again after it has stepped down. (Every completing warp used to
 // scan and race a CAS on the clock: with 21 ranges completed per us on an uncontended bank about
-// 50 scanned the same words at once, and completion took 13 to 38 us of a round.)
+// 50 scanned the same words at once, and completion took 13 to 38 us of a round; it takes 3.6.)
 static __device__ void complete_range(uint32_t* done, uint32_t done_mask, GlobalSync* gs, uint32_t lo,
                                uint32_t hi) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -369,26 +375,27 @@ static __device__ void complete_range(uint32_t* done, uint32_t done_mask, Global
   busy = __shfl_sync(FULL, busy, 0);
   if (busy) return;
   __syncwarp();
-  uint32_t c = ld_acquire_gpu(&gs->clock);  // only the advancing warp moves it
-  for (;;) {  // every pass moves the clock or steps down
-    const uint32_t n = complete_prefix(done, done_mask, c);
+  // the clock, and beside it the words where the scan starts when our range is the next
+  uint32_t c = ld_relaxed_gpu(&gs->clock), first = lo >> 5;
+  uint32_t w = ld_relaxed_gpu(&done[(first + lane) & done_mask]);
+  for (;;) {  // every pass moves the clock or leaves
+    const uint32_t n = complete_prefix(done, done_mask, c, first, w);
     __syncwarp();
     if (n != c) {
-      if (lane == 0) {
-        fence_acq_rel_gpu();
-        st_relaxed_gpu(&gs->clock, n);
-      }
-      // clear every word whose last timestamp this advance passed, for the next lap
+      // clear every word whose last timestamp this advance passes, for the next lap
       for (uint32_t wd = ((c + 1u) >> 5) + lane; wd * 32u + 31u <= n && wd <= (n >> 5); wd += 32u)
         st_relaxed_gpu(&done[wd & done_mask], 0u);
-      c = n;
-      continue;
+      __syncwarp();
     }
     if (lane == 0) {
       fence_acq_rel_gpu();
-      st_relaxed_gpu(&gs->advancing, 0u);
+      if (n != c) {
+        st_relaxed_gpu(&gs->clock, n);
+        fence_acq_rel_gpu();
+      }
+      st_relaxed_gpu(&gs->advancing, 0u);  // step down
       fence_sc_gpu();
-      const uint32_t t = c + 1u;  // the last look: the owner of c + 1 may have found us here
+      const uint32_t t = n + 1u;  // the last look: the owner of n + 1 may have found us here
       busy = (ld_relaxed_gpu(&done[(t >> 5) & done_mask]) >> (t & 31u)) & 1u
                  ? atomicExch(&gs->advancing, 1u)
                  : 1u;
@@ -400,6 +407,7 @@ static __device__ void complete_range(uint32_t* done, uint32_t done_mask, Global
     busy = __shfl_sync(FULL, busy, 0);
     if (busy) return;
     c = __shfl_sync(FULL, c, 0);
+    first = 0xFFFFFFFFu;  // (no words read ahead)
   }
 }
 
@@ -1113,6 +1121,231 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
 }
 
 // ---------------------------------------------------------------------------------------------
+// one transaction per commit (prevalidate 0 or 1, stamp protocol)
+// ---------------------------------------------------------------------------------------------
+
+// One attempt of a transfer round, warp-collective: read each account's latest committed version
+// with its stamp, lock the written accounts (lowest lane first, in address order, no waiting), drop
+// the lanes that read what a lower locked lane writes, draw timestamps from the commit server,
+// check that the stamps have not moved, install, publish the stamps. Returns the committed lanes.
+// *tried: locks were tried; *lost: one was held by another warp.
+// Bound by its chain of L2 round trips and fences (about 0.65 us a trip): loads that do not
+// depend on each other go out together, the victims' slots are read while the server draws, and
+// one pass over the candidates replaces the two all-pairs loops of TXWriteOverlap and
+// TXPreValidation (2.2 us).
+template <int DEPTH, int MAXR, int MAXW, bool CLUSTER>
+__device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm,
+                                  MailSlot<MAXR, MAXW>& ms, uint32_t me, uint32_t t, uint32_t op,
+                                  uint32_t nr, const uint32_t (&a)[MAXR], bool mine, uint32_t snap,
+                                  uint32_t& seq, bool& tried, bool& lost, bool& failed) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  const uint32_t lane = lane_id();
+  const VersionStore vs{p.slots, p.n_items};
+  // 1. latest versions and their stamps; a batch of reads in flight together
+  constexpr int kBatch = DEPTH <= 4 ? 4 : 2;
+  int32_t v[MAXR];
+  uint32_t stv[MAXR];
+  bool aborted = false;
+#pragma unroll
+  for (int k0 = 0; k0 < MAXR; k0 += kBatch) {
+    SlotEditor<DEPTH> e[kBatch]{};
+    unsigned long long w[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; j++)
+      w[j] = mine && k0 + j < (int)nr ? ld_relaxed_gpu(&p.cw[a[k0 + j]]) : 0ull;
+#pragma unroll
+    for (int j = 0; j < kBatch; j++)
+      if (mine && k0 + j < (int)nr) e[j].load(p.slots + (size_t)a[k0 + j] * DEPTH);
+#pragma unroll
+    for (int j = 0; j < kBatch; j++) {
+      const int k = k0 + j;
+      v[k] = 0;
+      stv[k] = (uint32_t)w[j];
+      // the stamp's version not visible yet (word and slots came together): the word again,
+      // then the slots after it
+      if (mine && k < (int)nr && !e[j].find(stv[k], v[k]))
+        aborted |= !read_latest<DEPTH>(vs, p.cw, a[k], stv[k], v[k]);
+    }
+  }
+  // 2. the transfer. One that writes nothing is read-only: it serialises at the largest stamp it
+  //    read, once a second collect finds every stamp unchanged and no lock on them (a writer of
+  //    one of them with a smaller timestamp would hold its lock)
+  int32_t w0 = 0, w1 = 0;
+  const bool has_w = mine && !aborted && transfer_writes<MAXR>(op, nr, v, w0, w1);
+  bool nowrite = mine && !aborted && !has_w;
+  uint32_t ro_snap = 0;
+  bool moved = false;
+#pragma unroll
+  for (int k = 0; k < MAXR; k++) {
+    if (!nowrite || k >= (int)nr) continue;
+    const unsigned long long wd = ld_relaxed_gpu(&p.cw[a[k]]);
+    moved |= (uint32_t)wd != stv[k] || (uint32_t)(wd >> 32) != 0u;
+    ro_snap = max(ro_snap, stv[k]);
+  }
+  const uint32_t stm = __ballot_sync(FULL, nowrite && moved);
+  nowrite = nowrite && !moved;
+  if (nowrite && p.log) {
+    p.outcome[t] = ro_snap | kSnapFlag;
+    p.result[t] = 0;
+  }
+  const uint32_t nwm = __ballot_sync(FULL, nowrite);
+  const uint32_t agm = __ballot_sync(FULL, mine && aborted);
+  uint32_t cand = __ballot_sync(FULL, has_w);
+  if (lane == 0) {
+    stat_add(sm.stat, ST_COMMIT_NOWRITE, __popc(nwm));
+    stat_add(sm.stat, ST_ABORT_DATA_AGE, __popc(agm));
+    stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(stm));
+  }
+  if (cand == 0u) return nwm;
+  // 3. lower candidates that write what this lane writes (overlap) or reads (conflict)
+  uint32_t overlap = 0, conflict = 0;
+  const uint32_t nr_max = __reduce_max_sync(FULL, has_w ? nr : 0u);
+  for (uint32_t m = cand; m & (m - 1u); m &= m - 1u) {  // (the highest has none above it)
+    const uint32_t i = __ffs(m) - 1u;
+    const uint32_t x0 = __shfl_sync(FULL, a[0], i), x1 = __shfl_sync(FULL, a[1], i);
+    const bool wr = a[0] == x0 || a[0] == x1 || a[1] == x0 || a[1] == x1;
+    bool rd = wr;
+#pragma unroll
+    for (int k = 2; k < MAXR; k++)
+      if (k < (int)nr_max) rd |= k < (int)nr && (a[k] == x0 || a[k] == x1);
+    const uint32_t bit = i < lane ? 1u << i : 0u;
+    overlap |= wr ? bit : 0u;
+    conflict |= rd ? bit : 0u;
+  }
+  // 4. locks first (before the timestamps are drawn; only the lowest lane writing an address
+  //    tries), then lane order among the lanes that hold their locks, so no lane is dropped for a
+  //    lower lane that could not lock. In address order, no waiting: the higher one is tried
+  //    only once the lower one is held, so two warps never each hold one of the other's pair
+  //    (that lock-step was a livelock); a lost lock releases what was taken and backs off.
+  const bool attempt = has_w && overlap == 0u;
+  const bool two = a[0] != a[1];
+  const uint32_t lo_a = min(a[0], a[1]), hi_a = max(a[0], a[1]);
+  bool got = false;
+  if (attempt) {
+    got = atomicCAS(owner_word(p.cw, lo_a), 0u, me) == 0u;
+    if (got && two && atomicCAS(owner_word(p.cw, hi_a), 0u, me) != 0u) {
+      st_relaxed_gpu(owner_word(p.cw, lo_a), 0u);
+      got = false;
+    }
+  }
+  const uint32_t locked = __ballot_sync(FULL, got);
+  tried = true;
+  lost = __any_sync(FULL, attempt && !got);
+  // a lane commits unless a lower committing lane of its own warp wrote what it read (their
+  // locks have the same owner): the lanes without a conflict do, the others in lane order
+  conflict &= locked;
+  uint32_t pass = __ballot_sync(FULL, got && conflict == 0u);
+  for (uint32_t m = locked & ~pass; m; m &= m - 1u)
+    pass |= __ballot_sync(FULL, lane == (uint32_t)__ffs(m) - 1u && (conflict & pass) == 0u);
+  if (got && !((pass >> lane) & 1u)) {
+    st_relaxed_gpu(owner_word(p.cw, lo_a), 0u);
+    if (two) st_relaxed_gpu(owner_word(p.cw, hi_a), 0u);
+  }
+  if (lane == 0) {
+    stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(cand & ~locked));
+    stat_add(sm.stat, p.prevalidate ? ST_ABORT_PREVALID : ST_ABORT_READ_WRITE, __popc(locked & ~pass));
+  }
+  cand = pass;
+  if (cand == 0u) return nwm;
+  const bool cand_me = (cand >> lane) & 1u;
+  // 5. post to the commit server; the locked accounts' slots are read while it draws (they stay
+  //    put while the locks are held)
+  seq++;
+  __syncwarp();
+  if (lane == 0) {
+    ms.snap = snap;
+    ms.cand = cand;
+    mail_release<CLUSTER>(&ms.req, seq);
+  }
+  uint32_t vic0 = 0, vic1 = 0;
+  {
+    fence_acq_rel_gpu();  // the previous holders' installs
+    SlotEditor<DEPTH> e0{}, e1{};
+    if (cand_me) e0.load(p.slots + (size_t)a[0] * DEPTH);
+    if (cand_me && two) e1.load(p.slots + (size_t)a[1] * DEPTH);
+    vic0 = e0.victim();
+    vic1 = e1.victim();
+  }
+  bool ok_wait = true;
+  if (lane == 0)
+    ok_wait = bounded_wait_fast([&] { return mail_acquire<CLUSTER>(&ms.rep) == seq; }, &p.gs->error,
+                                ERR_WAIT_REPLY, p.spin_log2);
+  ok_wait = __shfl_sync(FULL, ok_wait, 0);
+  if (!ok_wait) {
+    failed = true;
+    return nwm;
+  }
+  (void)mail_acquire<CLUSTER>(&ms.rep);
+  // 6. timestamps base+1.. in lane order, advertised in the lock words: a validator later in the
+  //    order may then ignore our lock, one earlier waits for our outcome instead of aborting.
+  //    (Every lane acquired the reply, which orders the validation after the draw.)
+  const uint32_t base = ms.base, my_ts = base + 1u + __popc(cand & lanemask_lt());
+  if (cand_me) {
+    st_relaxed_gpu(owner_word(p.cw, a[0]), kPendingFlag | my_ts);
+    if (two) st_relaxed_gpu(owner_word(p.cw, a[1]), kPendingFlag | my_ts);
+  }
+  // 7. validation: the stamps must not have moved, and a lock held by a transaction earlier in
+  //    the order (or one whose timestamp is not known yet) must be resolved first. Waits only
+  //    ever point to smaller timestamps: no cycles.
+  bool valid = cand_me;
+  if (cand_me) {
+    unsigned long long word[MAXR];
+#pragma unroll
+    for (int k = 0; k < MAXR; k++) word[k] = k < (int)nr ? ld_relaxed_gpu(&p.cw[a[k]]) : 0ull;
+#pragma unroll
+    for (int k = 0; k < MAXR; k++) {
+      if (k >= (int)nr || !valid) continue;
+      unsigned long long wd = word[k];
+      bool settled = false;
+      for (uint32_t it = 0; it < 2048; it++) {
+        const uint32_t own = (uint32_t)(wd >> 32);
+        if (own == 0u || own == me || ((own & kPendingFlag) && (own & ~kPendingFlag) >= my_ts)) {
+          settled = true;
+          break;
+        }
+        __nanosleep(32);
+        wd = ld_relaxed_gpu(&p.cw[a[k]]);
+      }
+      valid = settled && (uint32_t)wd == stv[k];
+    }
+  }
+  const uint32_t okm = __ballot_sync(FULL, valid);
+  if (lane == 0) {
+    stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(cand & ~okm));
+    stat_add(sm.stat, ST_COMMIT_UPDATE, __popc(okm));
+  }
+  // 8. install (a transfer writes a1 last: one of a single account keeps the credit), then the
+  //    stamps and the unlock, released by one fence; log; completion
+  if (valid) {
+    st_relaxed_gpu(p.slots + (size_t)a[0] * DEPTH + vic0, pack_version(my_ts, two ? w0 : w1));
+    if (two) st_relaxed_gpu(p.slots + (size_t)a[1] * DEPTH + vic1, pack_version(my_ts, w1));
+  }
+  fence_acq_rel_gpu();
+  if (cand_me) {
+    if (valid) {
+      st_relaxed_gpu(&p.cw[a[0]], (unsigned long long)my_ts);
+      if (two) st_relaxed_gpu(&p.cw[a[1]], (unsigned long long)my_ts);
+    } else {
+      st_relaxed_gpu(owner_word(p.cw, a[0]), 0u);
+      if (two) st_relaxed_gpu(owner_word(p.cw, a[1]), 0u);
+    }
+  }
+  if (p.log && cand_me) {
+    const uint32_t li = my_ts - 1u - p.log_base;
+    if (li < p.log_cap)
+      p.log_txn[li] = valid ? t : kHole;
+    else
+      raise_error(&p.gs->error, ERR_CAPACITY);
+    if (valid) {
+      p.outcome[t] = my_ts;
+      p.result[t] = 0;
+    }
+  }
+  complete_range(p.done, p.done_mask, p.gs, base + 1u, base + __popc(cand));
+  return nwm | okm;
+}
+
+// ---------------------------------------------------------------------------------------------
 // client side
 // ---------------------------------------------------------------------------------------------
 // CLUSTER: the mailbox `ms` (and the finished-client counter) live in the shared memory of the
@@ -1207,11 +1440,18 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
       const bool mine = (pending >> lane) & 1u;
       ReadSet<MAXR> rs;
       WriteSet<MAXW> ws;
-      uint32_t snap = 0;
-      if (lane == 0) snap = TXBegin(&p.gs->clock, rs, ws);
+      uint32_t snap = 0, err = 0;
+      if (lane == 0) {  // the device error word beside the clock: no round trip of its own
+        err = ld_relaxed_gpu(&p.gs->error);
+        snap = TXBegin(&p.gs->clock, rs, ws);
+      }
       rs.n = 0;
       ws.n = 0;
       snap = __shfl_sync(0xFFFFFFFFu, snap, 0);
+      if (__shfl_sync(0xFFFFFFFFu, err, 0) != 0u) {  // broadcast: the warp leaves the loop together
+        failed = true;
+        break;
+      }
       bool aborted = false;
 
       if (ro) {  // read-only: consistent snapshot read, commits without validation
@@ -1258,12 +1498,17 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
         }
         if (!gave_up) stuck = 0;
         pending &= ~fin;
-        uint32_t err = 0;
-        if (lane == 0) err = ld_relaxed_gpu(&p.gs->error);
-        if (__shfl_sync(0xFFFFFFFFu, err, 0) != 0) {
-          failed = true;
-          break;
-        }
+        continue;
+      }
+
+      if (stamp && p.prevalidate != 2) {  // one transaction per commit
+        bool lost = false, tried = false;
+        const uint32_t fin = stamp_attempt<DEPTH, MAXR, MAXW, CLUSTER>(
+            p, sm, ms, me, t, op, nr, a, mine, snap, seq, tried, lost, failed);
+        if (failed) break;
+        // back off only when a lock was lost to another warp (not for own-warp overlaps)
+        if (tried) lock_fails = lost ? min(lock_fails + 1, 6u) : 0u;
+        pending &= ~fin;
         continue;
       }
 
@@ -1283,7 +1528,6 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
             v[k] = TXRead<DEPTH>(vs, a[k], snap, rs, ws, &aborted);
         }
       }
-      const bool stale = false;
       // a transfer that commits no writes is read-only: in the stamp protocol it serialises at
       // the largest stamp it read, once a second collect finds every stamp unchanged and no
       // lock on them (a writer of one of them with a smaller timestamp would hold its lock)
@@ -1309,7 +1553,7 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
       // is locked once (by its lowest writer), and every link of the chain gets the next commit
       // timestamp. A link whose lock or validation fails takes down the links that consumed it.
       if (stamp && p.prevalidate == 2) {
-        const bool okr = mine && !aborted && !stale;
+        const bool okr = mine && !aborted;
         uint32_t dep = 0;  // lower lanes whose possible writes {a0, a1} hit my reads
         for (uint32_t i = 0; i < 31; i++) {
           const bool oki = __shfl_sync(0xFFFFFFFFu, okr, i);
@@ -1520,16 +1764,10 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
           stat_add(sm.stat, ST_COMMIT_NOWRITE, __popc(C & ~hw_c));
         }
         pending &= ~(C | snapm);
-        uint32_t err = 0;
-        if (lane == 0) err = ld_relaxed_gpu(&p.gs->error);
-        if (__shfl_sync(0xFFFFFFFFu, err, 0) != 0) {
-          failed = true;
-          break;
-        }
         continue;
       }
       bool has_w = false;
-      if (mine && !aborted && !stale) {
+      if (mine && !aborted) {
         uint32_t acc = CSMV_OP_AMT0(op) - 1u;
 #pragma unroll
         for (int k = 2; k < MAXR; k++)
@@ -1541,91 +1779,40 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
           has_w = true;
         }
       }
-      bool nowrite = mine && !aborted && !stale && !has_w;
-      bool ro_fail = false;
-      if (stamp) {
-        const bool ok = recheck(nowrite);
-        ro_fail = nowrite && !ok;
-        nowrite = nowrite && ok;
-      }
+      // ring protocol (the stamp protocol's modes have left above)
+      const bool nowrite = mine && !aborted && !has_w;
       if (nowrite && p.log) {
-        p.outcome[t] = ro_snap | kSnapFlag;
+        p.outcome[t] = snap | kSnapFlag;
         p.result[t] = 0;
       }
       const uint32_t nwm = __ballot_sync(0xFFFFFFFFu, nowrite);
       const uint32_t agm = __ballot_sync(0xFFFFFFFFu, mine && aborted);
-      const uint32_t stm = __ballot_sync(0xFFFFFFFFu, ro_fail);
       uint32_t cand = __ballot_sync(0xFFFFFFFFu, has_w);
       if (lane == 0) {
         stat_add(sm.stat, ST_COMMIT_NOWRITE, __popc(nwm));
         stat_add(sm.stat, ST_ABORT_DATA_AGE, __popc(agm));
-        stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(stm));
       }
       pending &= ~nwm;
       if (cand == 0) continue;
       bool cand_me = (cand >> lane) & 1u;
 
-      if (stamp) {
-        // lock the write items first (before the timestamps are drawn; only the lowest lane
-        // writing an address tries), then resolve lane order among the lanes that hold their
-        // locks, so no lane is dropped for a lower lane that could not lock
-        // (warp-collective: every lane calls it, candidate or not)
-        const uint32_t overlap = TXWriteOverlap(ws, cand_me);
-        const bool attempt = cand_me && (overlap & cand) == 0;
-        // locks in address order, no waiting: the higher one is tried only once the lower one is
-        // held, so two warps never each hold one of the other's pair (that lock-step was a
-        // livelock); a lost lock releases what was taken and backs off
-        static_assert(MAXW == 2, "ordered acquisition below is written for two write items");
-        const uint32_t lo_a = ws.n > 1 ? min(ws.addr[0], ws.addr[1]) : ws.addr[0];
-        const uint32_t hi_a = ws.n > 1 ? max(ws.addr[0], ws.addr[1]) : ws.addr[0];
-        bool got_lo = false, got_hi = ws.n < 2;
-        if (attempt) {
-          got_lo = atomicCAS(owner_word(p.cw, lo_a), 0u, me) == 0u;
-          if (got_lo && !got_hi) got_hi = atomicCAS(owner_word(p.cw, hi_a), 0u, me) == 0u;
-          if (got_lo && !got_hi) st_relaxed_gpu(owner_word(p.cw, lo_a), 0u);
-        }
-        const bool all = attempt && got_lo && got_hi;
-        bool got[MAXW];
-#pragma unroll
-        for (int k = 0; k < MAXW; k++) got[k] = all && k < (int)ws.n;
-        const uint32_t locked = __ballot_sync(0xFFFFFFFFu, all);
-        // intra-warp resolution: always needed here, since a lane must not commit after a lower
-        // lane of its own warp wrote what it read (their locks have the same owner)
-        const uint32_t pass = TXPreValidation(rs, ws, (locked >> lane) & 1u);
-        if (cand_me && !((pass >> lane) & 1u)) {
-#pragma unroll
-          for (int k = 0; k < MAXW; k++)
-            if (got[k]) st_relaxed_gpu(owner_word(p.cw, ws.addr[k]), 0u);
-        }
-        if (lane == 0) {
-          stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(cand & ~locked));
-          stat_add(sm.stat, p.prevalidate ? ST_ABORT_PREVALID : ST_ABORT_READ_WRITE,
-                   __popc(locked & ~pass));
-        }
-        // back off only when a lock was lost to another warp (not for own-warp overlaps)
-        lock_fails = __ballot_sync(0xFFFFFFFFu, attempt && !all) ? min(lock_fails + 1, 6u) : 0u;
+      if (p.prevalidate) {
+        const uint32_t pass = TXPreValidation(rs, ws, cand_me);
+        if (lane == 0) stat_add(sm.stat, ST_ABORT_PREVALID, __popc(cand & ~pass));
         cand = pass;
         cand_me = (cand >> lane) & 1u;
         if (cand == 0) continue;
-      } else {
-        if (p.prevalidate) {
-          const uint32_t pass = TXPreValidation(rs, ws, cand_me);
-          if (lane == 0) stat_add(sm.stat, ST_ABORT_PREVALID, __popc(cand & ~pass));
-          cand = pass;
-          cand_me = (cand >> lane) & 1u;
-          if (cand == 0) continue;
-        }
-        if (cand_me) {  // ring protocol: the server validates from the mailbox
+      }
+      if (cand_me) {  // ring protocol: the server validates from the mailbox
 #pragma unroll
-          for (int k = 0; k < MAXR; k++) ms.rs[k][lane] = rs.addr[k];
+        for (int k = 0; k < MAXR; k++) ms.rs[k][lane] = rs.addr[k];
 #pragma unroll
-          for (int k = 0; k < MAXW; k++) {
-            ms.ws[k][lane] = ws.addr[k];
-            ms.wv[k][lane] = ws.val[k];
-          }
-          ms.n[lane] = rs.n | (ws.n << 8);
-          ms.txn[lane] = t;
+        for (int k = 0; k < MAXW; k++) {
+          ms.ws[k][lane] = ws.addr[k];
+          ms.wv[k][lane] = ws.val[k];
         }
+        ms.n[lane] = rs.n | (ws.n << 8);
+        ms.txn[lane] = t;
       }
       // post the request into the shared-memory mailbox, wait for the reply
       seq++;
@@ -1646,95 +1833,22 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
       }
       (void)mail_acquire<CLUSTER>(&ms.rep);
 
-      uint32_t okm = 0, my_ts = 0;
-      if (stamp) {
-        // timestamps base+1.. in lane order over the locked lanes
-        const uint32_t base = ms.base;
-        my_ts = base + 1 + __popc(cand & lanemask_lt());
-        fence_acq_rel_gpu();
-        // advertise the pending timestamp in the lock words: a validator later in the order
-        // may then ignore our lock, one earlier waits for our outcome instead of aborting
-#pragma unroll
-        for (int k = 0; k < MAXW; k++)
-          if (cand_me && k < (int)ws.n) st_relaxed_gpu(owner_word(p.cw, ws.addr[k]), kPendingFlag | my_ts);
-        // validate the reads: the stamp must not be newer than the snapshot, and a lock held by
-        // a transaction earlier in the order (or one whose timestamp is not known yet) must be
-        // resolved first. Waits only ever point to smaller timestamps: no cycles.
-        bool valid = cand_me;
-        if (cand_me) {
-          unsigned long long word[MAXR];
-#pragma unroll
-          for (int k = 0; k < MAXR; k++)
-            word[k] = k < (int)rs.n ? ld_relaxed_gpu(&p.cw[rs.addr[k]]) : 0ull;
-#pragma unroll
-          for (int k = 0; k < MAXR; k++) {
-            if (k >= (int)rs.n || !valid) continue;
-            unsigned long long wd = word[k];
-            bool settled = false;
-            for (uint32_t it = 0; it < 2048; it++) {
-              const uint32_t own = (uint32_t)(wd >> 32);
-              if (own == 0u || own == me || ((own & kPendingFlag) && (own & ~kPendingFlag) >= my_ts)) {
-                settled = true;
-                break;
-              }
-              __nanosleep(32);
-              wd = ld_relaxed_gpu(&p.cw[rs.addr[k]]);
-            }
-            valid = settled && (uint32_t)wd == stv[k];
-          }
-        }
-        okm = __ballot_sync(0xFFFFFFFFu, valid);
-        if (lane == 0) stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(cand & ~okm));
-        if (p.log && cand_me) {
-          const uint32_t li = my_ts - 1 - p.log_base;
-          if (li < p.log_cap)
-            p.log_txn[li] = valid ? t : kHole;
-          else
-            raise_error(&p.gs->error, ERR_CAPACITY);
-        }
-        if (valid) {
-          TXWriteBack<DEPTH>(my_ts, vs, ws);
-          if (p.log) {
-            p.outcome[t] = my_ts;
-            p.result[t] = 0;
-          }
-        }
-        __threadfence();  // write-back visible before the stamps and the completion bits
-#pragma unroll
-        for (int k = 0; k < MAXW; k++) {
-          if (cand_me && k < (int)ws.n) {
-            if (valid)
-              st_release_gpu(&p.cw[ws.addr[k]], (unsigned long long)my_ts);  // stamp, unlock
-            else
-              st_relaxed_gpu(owner_word(p.cw, ws.addr[k]), 0u);
-          }
-        }
+      const uint32_t okm = ms.ok;
+      const uint32_t bid = ms.bid;
+      const bool committed = (okm >> lane) & 1u;
+      const uint32_t my_ts = committed ? ms.tsl[lane] : 0u;
+      if (committed && p.log) {
+        p.outcome[t] = my_ts;
+        p.result[t] = 0;
+      }
+      if (p.writeback == CSMV_WRITEBACK_CLIENT && okm) {
+        if (committed) TXWriteBack<DEPTH>(my_ts, vs, ws);
         __syncwarp();
-        complete_range(p.done, p.done_mask, p.gs, base + 1, base + __popc(cand));
-      } else {
-        okm = ms.ok;
-        const uint32_t bid = ms.bid;
-        const bool committed = (okm >> lane) & 1u;
-        my_ts = committed ? ms.tsl[lane] : 0u;
-        if (committed && p.log) {
-          p.outcome[t] = my_ts;
-          p.result[t] = 0;
-        }
-        if (p.writeback == CSMV_WRITEBACK_CLIENT && okm) {
-          if (committed) TXWriteBack<DEPTH>(my_ts, vs, ws);
-          __syncwarp();
-          if (lane == 0) batch_done(p, sm, bid);
-        }
+        if (lane == 0) batch_done(p, sm, bid);
       }
       __syncwarp();
       if (lane == 0) stat_add(sm.stat, ST_COMMIT_UPDATE, __popc(okm));
       pending &= ~okm;
-      uint32_t err = 0;  // read once and broadcast: the warp leaves the loop together
-      if (lane == 0) err = ld_relaxed_gpu(&p.gs->error);
-      if (__shfl_sync(0xFFFFFFFFu, err, 0) != 0) {
-        failed = true;
-        break;
-      }
     }
     if (failed) break;
     if (p.txn_aborts) p.txn_aborts[t] = tries - 1u;

@@ -485,3 +485,35 @@ def test_group_chain_sum_and_walk_equal_the_model(n_accounts, up_reads, amt, ini
     model = orc.sim_1warp(s.op, s.off, s.addr, n_accounts, np.full(n_accounts, init, np.int32), 4, 3)
     for got, want in zip((slots, log_txn, outcome, result), model):
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("prevalidate", [0, 1, 3])
+@pytest.mark.parametrize("up_reads,max_reads", [(2, 4), (2, 8), (4, 4), (8, 8)])
+def test_read_widths_on_one_warp_equal_the_model(up_reads, max_reads, prevalidate):
+    """Transfers of 2, 4 and 8 reads on one client warp, with funds that run short: log, outcomes,
+    results and versions equal the oracle's model. In group commit a transfer's accounts repeat
+    (a debit and a credit of one account among them; the model's other modes know distinct
+    accounts only)."""
+    rng = np.random.default_rng(up_reads * 10 + max_reads)
+    n_acc, rounds = 24, 40
+    n = 32 * rounds
+    ro = np.repeat(rng.random(rounds) < 0.2, 32)
+    op = np.where(ro, up_reads << 2 | 1 << 8 | 1 << 20,
+                  1 | up_reads << 2 | rng.integers(1, 8, n) << 8 | 7 << 20).astype(np.uint32)
+    off = (np.arange(n) * up_reads).astype(np.uint32)
+    if prevalidate == 3:
+        addr = rng.integers(0, n_acc, (n, up_reads))
+        same = rng.random(n) < 0.2
+        addr[same, 1] = addr[same, 0]
+    else:
+        addr = rng.permuted(np.tile(np.arange(n_acc), (n, 1)), axis=1)[:, :up_reads]
+    s = cg.Stream(op, off, np.ascontiguousarray(addr, np.uint32).reshape(-1))
+    init = np.full(n_acc, 60, np.int32)
+    model = orc.sim_1warp(s.op, s.off, s.addr, n_acc, init, 4, prevalidate)
+    with cg.Bank(n_accounts=n_acc, init_value=60, version_depth=4, ctas=1, client_warps=1, max_txn=n,
+                 prevalidate=prevalidate, max_reads=max_reads, batch=cg.BATCH_WARP) as bank:
+        bank.load()
+        st = bank.run(s)
+        log_txn, outcome, result = bank.log(n, st.final_ts)
+        for got, want in zip((bank.versions(), log_txn, outcome, result), model):
+            np.testing.assert_array_equal(got, want)
