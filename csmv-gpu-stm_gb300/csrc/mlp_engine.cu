@@ -20,6 +20,12 @@ struct csmv_mlp_t {
   cudaStream_t stream = nullptr;
   float *master = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr, *loss = nullptr;
   __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
+  unsigned char* wimg = nullptr;   // weights and biases as the inference kernel's operands
+  // Host word that the inference kernel writes when a wait of it runs out: this one, where the
+  // device reads and writes any host memory (a coherent CPU link), else a mapped allocation
+  // (which costs 300 us to make).
+  alignas(64) uint32_t fail_word = 0;
+  uint32_t *fail = nullptr, *fail_dev = nullptr;
   uint32_t steps = 0;
 };
 
@@ -33,6 +39,8 @@ void free_all(csmv_mlp_t* h) {
   cudaFree(h->w1);
   cudaFree(h->w2);
   cudaFree(h->w3);
+  cudaFree(h->wimg);
+  if (h->fail && h->fail != &h->fail_word) cudaFreeHost(h->fail);
   if (h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -66,9 +74,22 @@ extern "C" csmv_status csmv_mlp_create(int32_t device, uint64_t seed, csmv_mlp_t
   } allocs[] = {{(void**)&h->master, pb}, {(void**)&h->grad, pb}, {(void**)&h->m, pb},
                 {(void**)&h->v, pb}, {(void**)&h->loss, 16},
                 {(void**)&h->w1, kMlpIn * kMlpHid * 2}, {(void**)&h->w2, kMlpHid * kMlpHid * 2},
-                {(void**)&h->w3, kMlpHid * 2}};
+                {(void**)&h->w3, kMlpHid * 2}, {(void**)&h->wimg, kTcImageBytes}};
   for (auto& a : allocs)
     if ((st = cuda_status(cudaMalloc(a.p, a.bytes), "cudaMalloc")) != CSMV_OK) return fail(st);
+  int any_host = 0;
+  if ((st = cuda_status(cudaDeviceGetAttribute(&any_host, cudaDevAttrPageableMemoryAccess, device),
+                        "cudaDeviceGetAttribute")) != CSMV_OK)
+    return fail(st);
+  if (any_host) {
+    h->fail = h->fail_dev = &h->fail_word;
+  } else {
+    if ((st = cuda_status(cudaHostAlloc((void**)&h->fail, 4, cudaHostAllocMapped), "cudaHostAlloc")) != CSMV_OK ||
+        (st = cuda_status(cudaHostGetDevicePointer((void**)&h->fail_dev, h->fail, 0),
+                          "cudaHostGetDevicePointer")) != CSMV_OK)
+      return fail(st);
+    *h->fail = 0u;
+  }
   if ((st = cuda_status(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream")) != CSMV_OK)
     return fail(st);
   if ((st = cuda_status(cudaFuncSetAttribute((const void*)mlp_grad_kernel,
@@ -77,7 +98,7 @@ extern "C" csmv_status csmv_mlp_create(int32_t device, uint64_t seed, csmv_mlp_t
                         "cudaFuncSetAttribute")) != CSMV_OK ||
       (st = cuda_status(cudaFuncSetAttribute((const void*)mlp_forward_tc_kernel,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(MlpTcSmem)),
+                                             (int)kTcSmemBytes),
                         "cudaFuncSetAttribute")) != CSMV_OK)
     return fail(st);
   // uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) weights, zero biases
@@ -105,7 +126,8 @@ extern "C" csmv_status csmv_mlp_set_params(csmv_mlp_t* h, const float* host_para
   CSMV_CUDA(cudaMemsetAsync(h->grad, 0, pb, h->stream));
   CSMV_CUDA(cudaMemsetAsync(h->m, 0, pb, h->stream));
   CSMV_CUDA(cudaMemsetAsync(h->v, 0, pb, h->stream));
-  mlp_round_weights_kernel<<<32, 256, 0, h->stream>>>(h->master, h->w1, h->w2, h->w3);
+  CSMV_CUDA(cudaMemsetAsync(h->wimg, 0, kTcImageBytes, h->stream));
+  mlp_round_weights_kernel<<<32, 256, 0, h->stream>>>(h->master, h->w1, h->w2, h->w3, h->wimg);
   CSMV_CUDA(cudaGetLastError());
   CSMV_CUDA(cudaStreamSynchronize(h->stream));
   h->steps = 0;
@@ -130,11 +152,11 @@ extern "C" csmv_status csmv_mlp_get_grads(csmv_mlp_t* h, float* host_grads) {
 csmv_status csmv_mlp_launch_forward(csmv_mlp_t* h, uint32_t n, const void* dev_x, float* dev_p,
                                     cudaStream_t stream) {
   if (n == 0) return CSMV_OK;
-  // two 104 KB CTAs per SM
-  const uint32_t tiles = (n + kTcTile - 1) / kTcTile, cap = 2u * (uint32_t)h->n_sms;
-  const uint32_t grid = tiles < cap ? tiles : cap;
-  mlp_forward_tc_kernel<<<grid, 256, sizeof(MlpTcSmem), stream>>>(
-      static_cast<const __nv_bfloat16*>(dev_x), n, h->w1, h->w2, h->w3, h->master, dev_p);
+  // one CTA per SM; a tile goes to the first group of each CTA before any second one
+  const uint32_t tiles = (n + kTcTile - 1) / kTcTile;
+  const uint32_t grid = tiles < (uint32_t)h->n_sms ? tiles : (uint32_t)h->n_sms;
+  mlp_forward_tc_kernel<<<grid, kTcThreads, kTcSmemBytes, stream>>>(
+      static_cast<const __nv_bfloat16*>(dev_x), n, h->wimg, h->w3, h->master, dev_p, h->fail_dev);
   return cuda_status(cudaGetLastError(), "mlp_forward_tc_kernel");
 }
 
@@ -154,11 +176,19 @@ csmv_status csmv_mlp_launch_adam(csmv_mlp_t* h, float lr, cudaStream_t stream) {
   h->steps++;
   const float b1t = (float)std::pow(0.9, (double)h->steps), b2t = (float)std::pow(0.999, (double)h->steps);
   mlp_adam_kernel<<<32, 256, 0, stream>>>(h->master, h->grad, h->m, h->v, lr, b1t, b2t, h->w1,
-                                          h->w2, h->w3);
+                                          h->w2, h->w3, h->wimg);
   return cuda_status(cudaGetLastError(), "mlp_adam_kernel");
 }
 
 float* csmv_mlp_loss_ptr(csmv_mlp_t* h) { return h->loss; }
+
+// After the stream of a forward launch is idle: did one of its bounded waits run out?
+csmv_status csmv_mlp_forward_status(csmv_mlp_t* h) {
+  if (*reinterpret_cast<volatile uint32_t*>(h->fail) == 0u) return CSMV_OK;
+  *h->fail = 0u;
+  set_error("mlp_forward_tc_kernel: a wait for the tensor cores ran out");
+  return CSMV_ERR_TIMEOUT;
+}
 
 extern "C" csmv_status csmv_mlp_forward(csmv_mlp_t* h, uint32_t n, const uint16_t* dev_x,
                                         float* dev_p) {
@@ -167,7 +197,7 @@ extern "C" csmv_status csmv_mlp_forward(csmv_mlp_t* h, uint32_t n, const uint16_
   csmv_status st = csmv_mlp_launch_forward(h, n, dev_x, dev_p, h->stream);
   if (st != CSMV_OK) return st;
   CSMV_CUDA(cudaStreamSynchronize(h->stream));
-  return CSMV_OK;
+  return csmv_mlp_forward_status(h);
 }
 
 extern "C" csmv_status csmv_mlp_grad(csmv_mlp_t* h, uint32_t n, const uint16_t* dev_x,

@@ -26,6 +26,7 @@ csmv_status csmv_mlp_launch_grad(csmv_mlp_t* h, uint32_t n, const void* dev_x, c
                                  cudaStream_t stream);
 csmv_status csmv_mlp_launch_adam(csmv_mlp_t* h, float lr, cudaStream_t stream);
 float* csmv_mlp_loss_ptr(csmv_mlp_t* h);
+csmv_status csmv_mlp_forward_status(csmv_mlp_t* h);
 
 struct csmv_sched_t {
   csmv_sched_config cfg{};
@@ -282,6 +283,7 @@ extern "C" csmv_status csmv_sched_plan_run(csmv_sched_t* s, csmv_bank_t* bank,
   uint32_t r_ro = 0;
   CSMV_CUDA(cudaMemcpyAsync(&r_ro, s->ro_scan + Rp, 4, cudaMemcpyDeviceToHost, s->stream));
   CSMV_CUDA(cudaStreamSynchronize(s->stream));
+  if ((st = csmv_mlp_forward_status(s->mlp)) != CSMV_OK) return st;
   const uint32_t U = Rp - r_ro;  // transfer rounds
   uint32_t flagged = 0, deferred_rounds = 0;
   const uint32_t* run_op = d->op + t0;

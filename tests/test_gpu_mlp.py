@@ -102,3 +102,43 @@ def test_training_learns_a_separable_labelling():
         m.forward(20000, dx.data_ptr(), dp.data_ptr())
         acc = float(((dp.cpu().numpy() > 0.5) == (y > 0.5)).mean())
     assert loss < 0.25 * first and acc > 0.97, (first, loss, acc)
+
+
+@pytest.mark.parametrize("n", [31, 127, 128, 129, 152 * 128, 152 * 128 + 1, 2 * 152 * 128 + 77,
+                               5 * 152 * 128 + 130])
+def test_forward_at_tile_and_grid_edges(n):
+    """Inference over partial and whole tiles of 128, one to several tiles a group of the grid's
+    CTAs, with biases that do not fit one bf16: probabilities match the float64 oracle, and
+    nothing beyond n is written. With such biases a layer-1 sum can round to the neighbouring
+    bf16 value, as for dense features above: 2e-4 absolute, 2e-5 for all but 1e-3 of the samples."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    x, xb = _features(rng, n)
+    with cg.Mlp(seed=11) as m:
+        params = m.params()
+        params[mo.OFF_B1:mo.OFF_W2] = rng.normal(0, 0.4, mo.HID)
+        params[mo.OFF_B2:mo.OFF_W3] = rng.normal(0, 0.4, mo.HID)
+        params[mo.OFF_B3] = -0.2
+        m.set_params(params)
+        dx, dp = _dev(torch, xb), torch.full((n + 256,), 7.0, device="cuda")
+        m.forward(n, dx.data_ptr(), dp.data_ptr())
+        p = dp.cpu().numpy()
+    off = np.abs(p[:n] - mo.forward(params, x)[0])
+    assert off.max() <= 2e-4 and np.mean(off > 2e-5) < 1e-3
+    assert (p[n:] == 7.0).all()
+
+
+def test_forward_after_training_uses_the_new_weights():
+    """The inference operands follow Adam's updates of weights and biases."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(2)
+    x, xb = _features(rng, 700)
+    y = (x[:, 5] > 0).astype(np.float32)
+    with cg.Mlp(seed=3) as m:
+        dx, dy = _dev(torch, xb), _dev(torch, y)
+        dp = torch.zeros(700, device="cuda")
+        for _ in range(5):
+            m.grad(700, dx.data_ptr(), dy.data_ptr())
+            m.adam_step(1e-2)
+        m.forward(700, dx.data_ptr(), dp.data_ptr())
+        np.testing.assert_allclose(dp.cpu().numpy(), mo.forward(m.params(), x)[0], rtol=0, atol=2e-5)
