@@ -15,10 +15,17 @@
 // used only if its tag did not move (a sequence-lock). The tags of a set's 8 ways sit in one
 // 128-byte line: a GET at snapshot S loads them in one access, picks per way the newest version
 // <= S, and reads only the records whose valid hash matches, in way order (first full key match
-// wins, as the reference breaks at the first match). A SET reads each way's latest committed
+// wins, as the reference breaks at the first match). A SET looks at each way's latest committed
 // version (by its commit word), chooses the slot by the reference's rule, locks only that entry,
 // takes a commit timestamp from the CTA's server, validates the eight stamps and installs the
 // new version. Rounds of 32 requests are warp-uniform GETs or SETs (memcdSH.cu:333-339).
+//
+// Bound under Zipf(0.99) by the hottest entry's lock, through which its SETs pass one hold after
+// the other, and by the GETs that wait for holders. A warp's SETs of one key therefore share a
+// hold; a hold is kept to the timestamp draw, the validation and three fences; and records
+// are read only where a tag's hash says so. A batch of 64 K requests with 1 % SETs on 2^20 sets
+// took 2.3 ms before that and takes 0.21 ms; a serving session of 495 K requests with 5 % SETs
+// took 57 ms and takes 5.1 ms.
 #pragma once
 #include <cstdint>
 
@@ -29,6 +36,7 @@ namespace csmv {
 constexpr int kWays = 8;
 constexpr int kMemcdDepth = 2;
 constexpr uint32_t kValidBit = 0x80000000u;
+constexpr uint32_t kMemcdBackoffLog2 = 6;  // longest pause after lost locks: 64 << this (ns)
 
 struct MemcdParams {
   const uint32_t* kind;  // [n] 0 = GET, 1 = SET
@@ -99,6 +107,8 @@ __device__ __forceinline__ uint32_t tag_ts(unsigned long long t) { return (uint3
 __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms, uint32_t me,
                             uint32_t r, uint32_t& seq, uint32_t tick) {
   constexpr int D = kMemcdDepth;
+  static_assert(D == 2, "two versions an entry");
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = lane_id();
   bool failed = false;
   {
@@ -130,24 +140,24 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
         __nanosleep((h >> 16) & ((64u << lock_fails) - 1u));
       }
       const bool mine = (pending >> lane) & 1u;
-      uint32_t snap = 0;
-      if (lane == 0) snap = ld_acquire_gpu(&p.gs->clock);
-      snap = __shfl_sync(0xFFFFFFFFu, snap, 0);
-      // the set's tag words: 8 ways x kMemcdDepth versions, one 128-byte line
-      unsigned long long tg[kWays * D];
-      if (mine) {
-#pragma unroll
-        for (int i = 0; i < kWays * D; i += 2)
-          ld_relaxed_gpu_v2(p.tag + (size_t)e0 * D + i, tg[i], tg[i + 1]);
+      uint32_t snap = 0, err = 0;
+      if (lane == 0) {  // the device error word beside the clock
+        err = ld_relaxed_gpu(&p.gs->error);
+        snap = ld_acquire_gpu(&p.gs->clock);
+      }
+      snap = __shfl_sync(FULL, snap, 0);
+      if (__shfl_sync(FULL, err, 0) != 0u) {
+        failed = true;
+        break;
       }
 
       if (!is_set) {
         // GET: the latest committed version of each way, read through its commit word and
         // re-checked afterwards (a double collect), serialised at the largest stamp read. The
-        // stamp's version is never a writer's victim (that is the older slot), so its record
-        // stays put while the stamp does. Locks: a holder with a timestamp above the snapshot
-        // commits after it and is ignored; one below it, or one still without a timestamp when
-        // the GET looks, may commit inside the snapshot, so the GET waits (bounded) or retries.
+        // record read is checked by its tag too (several SETs of one key that commit together
+        // replace both versions). Locks: a holder with a timestamp above the snapshot commits
+        // after it and is ignored; one below it makes the GET retry; one still without a
+        // timestamp when the GET looks may commit inside the snapshot and is waited for (bounded).
         bool found = false, aged = false;
         uint32_t smax = 0;
         uint4 o0 = make_uint4(0, 0, 0, 0), o1 = o0;
@@ -157,58 +167,50 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
           for (int wy = 0; wy < kWays; wy++) w1[wy] = ld_relaxed_gpu(&p.cw[e0 + wy]);
 #pragma unroll
           for (int wy = 0; wy < kWays; wy++) {
-            // a holder still without a timestamp is waited for (bounded); so, briefly, is one
-            // with a timestamp (a SET about to install: waiting for it costs less than the
-            // retry its timestamp below the snapshot would force)
             for (uint32_t it = 0; it < 512u; it++) {
               const uint32_t own = (uint32_t)(w1[wy] >> 32);
-              if (own == 0u || ((own & kPendingFlag) && it >= 32u)) break;
+              if (own == 0u || (own & kPendingFlag)) break;
               __nanosleep(64);
               w1[wy] = ld_relaxed_gpu(&p.cw[e0 + wy]);
             }
           }
           fence_acq_rel_gpu();  // versions after the stamps
-          unsigned long long tg2[kWays * D];
+          unsigned long long tg[kWays * D];
 #pragma unroll
           for (int i = 0; i < kWays * D; i += 2)
-            ld_relaxed_gpu_v2(p.tag + (size_t)e0 * D + i, tg2[i], tg2[i + 1]);
-          int pick[kWays];
-          unsigned long long ptag[kWays];
+            ld_relaxed_gpu_v2(p.tag + (size_t)e0 * D + i, tg[i], tg[i + 1]);
+          uint32_t hit = 0, second = 0;  // ways whose latest version has the key's hash; its slot
 #pragma unroll
           for (int wy = 0; wy < kWays; wy++) {
             const uint32_t st = (uint32_t)w1[wy], own = (uint32_t)(w1[wy] >> 32);
             if (own != 0u && !(own & kPendingFlag)) aged = true;  // still no timestamp: retry
             smax = max(smax, st);
-            int j = -1;
-            unsigned long long t0 = 0;
+            bool there = false;
 #pragma unroll
             for (int q = 0; q < D; q++)
-              if (tag_ts(tg2[wy * D + q]) == st) {
-                j = q;
-                t0 = tg2[wy * D + q];
+              if (tag_ts(tg[wy * D + q]) == st) {
+                there = true;
+                second |= (uint32_t)q << wy;
+                if ((uint32_t)tg[wy * D + q] == th) hit |= 1u << wy;
               }
-            pick[wy] = j;
-            ptag[wy] = t0;
-            aged |= j < 0;
+            aged |= !there;
           }
 #pragma unroll
           for (int wy = 0; wy < kWays; wy++) {
             const uint32_t own = (uint32_t)(w1[wy] >> 32);
             if ((own & kPendingFlag) && (own & ~kPendingFlag) < smax) aged = true;
           }
-#pragma unroll
-          for (int wy = 0; wy < kWays; wy++) {
-            const unsigned long long t0 = ptag[wy];
-            // skip: decided, or not valid, or another key's hash
-            if (aged || found || (uint32_t)t0 != th) continue;
-            const size_t v = (size_t)(e0 + wy) * D + pick[wy];
+          uint32_t read = 0;  // ways whose record was read
+          for (uint32_t m = aged ? 0u : hit; m && !found; m &= m - 1u) {
+            const uint32_t wy = __ffs(m) - 1u;
+            const size_t v = (size_t)(e0 + wy) * D + ((second >> wy) & 1u);
+            read |= 1u << wy;
             const uint4 kk = ld_relaxed_gpu_v4(p.rec + v * 4 + 1);
-            if (key_eq(kk, key)) {
-              found = true;
-              o0 = ld_relaxed_gpu_v4(p.rec + v * 4 + 2);
-              o1 = ld_relaxed_gpu_v4(p.rec + v * 4 + 3);
-            }
+            o0 = ld_relaxed_gpu_v4(p.rec + v * 4 + 2);
+            o1 = ld_relaxed_gpu_v4(p.rec + v * 4 + 3);
+            found = key_eq(kk, key);
           }
+          if (!found) o0 = o1 = make_uint4(0, 0, 0, 0);
           fence_acq_rel_gpu();
 #pragma unroll
           for (int wy = 0; wy < kWays; wy++) {  // the second collect
@@ -218,6 +220,15 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
             if ((own & kPendingFlag) && (own & ~kPendingFlag) < smax) aged = true;
             // a holder without a timestamp that locked after the first collect draws its
             // timestamp after every stamp read here: it lands above the snapshot
+          }
+          for (uint32_t m = read; m; m &= m - 1u) {
+            const uint32_t wy = __ffs(m) - 1u;
+            const unsigned long long t2 =
+                ld_relaxed_gpu(p.tag + (size_t)(e0 + wy) * D + ((second >> wy) & 1u));
+            uint32_t st = 0;
+#pragma unroll
+            for (int q = 0; q < kWays; q++) st = wy == (uint32_t)q ? (uint32_t)w1[q] : st;
+            if (tag_ts(t2) != st) aged = true;  // the record was being replaced
           }
         }
         const bool done = mine && !aged;
@@ -229,8 +240,8 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
           // the state read is also the state at that clock when it is the later of the two
           if (p.log) p.outcome[r] = max(smax, snap) | kSnapFlag;
         }
-        const uint32_t dm = __ballot_sync(0xFFFFFFFFu, done);
-        const uint32_t am = __ballot_sync(0xFFFFFFFFu, mine && aged);
+        const uint32_t dm = __ballot_sync(FULL, done);
+        const uint32_t am = __ballot_sync(FULL, mine && aged);
         if (lane == 0) {
           stat_add(sm.stat, ST_COMMIT_RO, __popc(dm));
           stat_add(sm.stat, ST_ABORT_DATA_AGE, __popc(am));
@@ -239,102 +250,123 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
         continue;
       }
 
-      // SET: each way's latest committed version (the one whose ts is the way's stamp); the
-      // slot by the reference's rule: the way holding the key (valid), else the smallest LRU
-      // timestamp, first on ties (memcdSH.cu:365-387)
+      // SET. The warp's SETs of one key commit together: their lowest lane reads the set, locks
+      // the entry and validates for all of them, and they take timestamps in lane order; of the
+      // versions they would install one after the other only the last two remain, and only
+      // those are written. (Under Zipf(0.99) the hottest key's SETs follow each other through one
+      // lock, two of a round's 32 on average.) When lanes with different keys share a set, only
+      // the lowest of them takes part this time.
+      const uint32_t peers = __match_any_sync(FULL, mine ? e0 : 0x80000000u | lane);
+      const uint32_t lead = __ffs(peers) - 1u;
+      const uint4 lk = make_uint4(__shfl_sync(FULL, key.x, lead), __shfl_sync(FULL, key.y, lead),
+                                  __shfl_sync(FULL, key.z, lead), __shfl_sync(FULL, key.w, lead));
+      const uint32_t samem = __ballot_sync(FULL, key_eq(lk, key));
+      const bool leader = mine && lane == lead;
+      const bool member = mine && (leader || (peers & ~samem) == 0u);
+      // the leader reads each way's latest committed version (the one whose ts is the way's
+      // stamp) and picks the slot by the reference's rule: the way holding the key (valid), else
+      // the smallest LRU timestamp, first on ties (memcdSH.cu:365-387). Records are read only
+      // where the tag's hash matches or, without a match, for the LRU timestamps.
       uint32_t stw[kWays];
+      unsigned long long pick[kWays];  // tag of each way's latest version
+      unsigned long long other = 0;    // tag of the target's other version
+      uint32_t second = 0, used = 0;   // slot of the latest version; ways whose record was read
       bool aborted = false;
-      int slot = -1;
-      uint32_t slot_lru = 0;
-      bool matched = false;
+      int slot = 0;
 #pragma unroll
-      for (int wy = 0; wy < kWays; wy++) stw[wy] = 0;
-      if (mine) {
-        unsigned long long wordv[kWays];
+      for (int wy = 0; wy < kWays; wy++) {
+        stw[wy] = 0;
+        pick[wy] = 0;
+      }
+      if (leader) {
+        unsigned long long tg[kWays * D];
 #pragma unroll
-        for (int wy = 0; wy < kWays; wy++) wordv[wy] = ld_relaxed_gpu(&p.cw[e0 + wy]);
-        fence_acq_rel_gpu();  // the record loads stay behind the tag loads (sequence lock)
-        int sj[kWays];
-        unsigned long long s0[kWays];
-        uint32_t lru[kWays];
-        bool km[kWays];
-#pragma unroll
-        for (int wy = 0; wy < kWays; wy++) {
-          const uint32_t st = (uint32_t)wordv[wy];
-          stw[wy] = st;
-          int j = -1;
-          unsigned long long t0 = 0;
-#pragma unroll
-          for (int q = 0; q < D; q++)
-            if (tag_ts(tg[wy * D + q]) == st) {
-              j = q;
-              t0 = tg[wy * D + q];
-            }
-          sj[wy] = j;
-          s0[wy] = t0;
-          lru[wy] = 0;
-          km[wy] = false;
-          if (j < 0) {  // the stamp's version not seen yet (fetched concurrently): retry
-            aborted = true;
-            continue;
-          }
-          const size_t v = (size_t)(e0 + wy) * D + j;
-          const uint4 hd = ld_relaxed_gpu_v4(p.rec + v * 4);
-          const uint4 kk = ld_relaxed_gpu_v4(p.rec + v * 4 + 1);
-          lru[wy] = hd.x;
-          km[wy] = ((uint32_t)t0 & kValidBit) && key_eq(kk, key);
-        }
-        fence_acq_rel_gpu();
-        unsigned long long tg2[kWays * D];
+        for (int wy = 0; wy < kWays; wy++) stw[wy] = (uint32_t)ld_relaxed_gpu(&p.cw[e0 + wy]);
+        fence_acq_rel_gpu();  // versions after the stamps
 #pragma unroll
         for (int i = 0; i < kWays * D; i += 2)
-          ld_relaxed_gpu_v2(p.tag + (size_t)e0 * D + i, tg2[i], tg2[i + 1]);
+          ld_relaxed_gpu_v2(p.tag + (size_t)e0 * D + i, tg[i], tg[i + 1]);
+        uint32_t hit = 0;
 #pragma unroll
         for (int wy = 0; wy < kWays; wy++) {
+          bool there = false;
 #pragma unroll
           for (int q = 0; q < D; q++)
-            if (q == sj[wy] && tg2[wy * D + q] != s0[wy]) aborted = true;  // record moved
-          if (!matched) {
-            if (km[wy]) {
-              slot = wy;
-              matched = true;
-            } else if (slot < 0 || lru[wy] < slot_lru) {
-              slot = wy;
-              slot_lru = lru[wy];
+            if (tag_ts(tg[wy * D + q]) == stw[wy]) {
+              there = true;
+              second |= (uint32_t)q << wy;
+              pick[wy] = tg[wy * D + q];
+              if ((uint32_t)pick[wy] == th) hit |= 1u << wy;
             }
-          }
+          aborted |= !there;  // being replaced: retry
+        }
+        fence_acq_rel_gpu();  // the record loads stay behind the tag loads (sequence lock)
+        bool matched = false;
+        for (uint32_t m = aborted ? 0u : hit; m && !matched; m &= m - 1u) {
+          const uint32_t wy = __ffs(m) - 1u;
+          used |= 1u << wy;
+          matched = key_eq(ld_relaxed_gpu_v4(p.rec + ((size_t)(e0 + wy) * D + ((second >> wy) & 1u)) * 4 + 1), key);
+          if (matched) slot = (int)wy;
+        }
+        if (!matched && !aborted) {
+          uint32_t lru[kWays];
+#pragma unroll
+          for (int wy = 0; wy < kWays; wy++)
+            lru[wy] = ld_relaxed_gpu(reinterpret_cast<const uint32_t*>(
+                p.rec + ((size_t)(e0 + wy) * D + ((second >> wy) & 1u)) * 4));
+#pragma unroll
+          for (int wy = 1; wy < kWays; wy++)
+            if (lru[wy] < lru[0]) {
+              lru[0] = lru[wy];
+              slot = wy;
+            }
+          used = 0xFFu;
+        }
+#pragma unroll
+        for (int wy = 0; wy < kWays; wy++)
+          if (wy == slot) other = tg[wy * D + ((second >> wy) & 1u ? 0 : 1)];
+        fence_acq_rel_gpu();
+      }
+      // the lock, by a CAS that also proves the entry's stamp (so its versions are the ones
+      // read), beside a second look at the tags: no record that was read has been replaced
+      uint32_t target = e0 + (uint32_t)slot, st0 = 0;
+      bool got = false;
+      if (leader && !aborted) {
+#pragma unroll
+        for (int wy = 0; wy < kWays; wy++) st0 = wy == slot ? stw[wy] : st0;
+        unsigned long long t2[kWays];
+#pragma unroll
+        for (int wy = 0; wy < kWays; wy++)
+          t2[wy] = (used >> wy) & 1u ? ld_relaxed_gpu(p.tag + (size_t)(e0 + wy) * D + ((second >> wy) & 1u)) : pick[wy];
+        const unsigned long long free_w = st0;
+        got = atomicCAS(&p.cw[target], free_w, free_w | ((unsigned long long)me << 32)) == free_w;
+        bool moved = false;
+#pragma unroll
+        for (int wy = 0; wy < kWays; wy++) moved |= t2[wy] != pick[wy];
+        if (moved) {
+          if (got) st_relaxed_gpu(&p.cw[target], free_w);
+          got = false;
+          aborted = true;
         }
       }
-      const uint32_t target = e0 + (uint32_t)(slot < 0 ? 0 : slot);
-      // intra-warp: lane order over (reads: the 8 entries of the set, write: the slot)
-      ReadSet<kWays> rs;
-      WriteSet<1> ws;
-      bool cand_me = mine && !aborted;
-      if (cand_me) {
-        rs.n = kWays;
-#pragma unroll
-        for (int wy = 0; wy < kWays; wy++) rs.addr[wy] = e0 + wy;
-        ws.n = 1;
-        ws.addr[0] = target;
+      const uint32_t locked = __ballot_sync(FULL, got);
+      const uint32_t agedm = __ballot_sync(FULL, leader && aborted);
+      const bool cand_me = member && ((locked >> lead) & 1u);
+      const uint32_t cand = __ballot_sync(FULL, cand_me);
+      {
+        const uint32_t agm = __ballot_sync(FULL, member && ((agedm >> lead) & 1u));
+        const uint32_t wwm = __ballot_sync(FULL, member && !cand_me && !((agedm >> lead) & 1u));
+        const uint32_t pvm = __ballot_sync(FULL, mine && !member);
+        if (lane == 0) {
+          stat_add(sm.stat, ST_ABORT_DATA_AGE, __popc(agm));
+          stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(wwm));
+          stat_add(sm.stat, ST_ABORT_PREVALID, __popc(pvm));
+        }
+        lock_fails = wwm ? min(lock_fails + 1, kMemcdBackoffLog2) : 0u;
       }
-      uint32_t cand = __ballot_sync(0xFFFFFFFFu, cand_me);
-      const uint32_t overlap = TXWriteOverlap(ws, cand_me);
-      const bool attempt = cand_me && (overlap & cand) == 0;
-      const bool got = attempt && atomicCAS(owner_word(p.cw, target), 0u, me) == 0u;
-      const uint32_t locked = __ballot_sync(0xFFFFFFFFu, got);
-      const uint32_t pass = TXPreValidation(rs, ws, got);
-      if (got && !((pass >> lane) & 1u)) st_relaxed_gpu(owner_word(p.cw, target), 0u);
-      const uint32_t agm = __ballot_sync(0xFFFFFFFFu, mine && aborted);
-      if (lane == 0) {
-        stat_add(sm.stat, ST_ABORT_DATA_AGE, __popc(agm));
-        stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(cand & ~locked));
-        stat_add(sm.stat, ST_ABORT_PREVALID, __popc(locked & ~pass));
-      }
-      lock_fails = __ballot_sync(0xFFFFFFFFu, attempt && !got) ? min(lock_fails + 1, 6u) : 0u;
-      cand = pass;
-      cand_me = (cand >> lane) & 1u;
       if (cand == 0) continue;
-      // commit timestamps from the CTA's server
+      // commit timestamps from the CTA's server; meanwhile the version to replace is withdrawn
+      // (the older one: no reader uses it)
       seq++;
       __syncwarp();
       if (lane == 0) {
@@ -342,28 +374,43 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
         ms.cand = cand;
         st_release_cta(&ms.req, seq);
       }
+      const uint32_t group = peers & cand, n_group = __popc(group), rank = __popc(group & lanemask_lt());
+      target = __shfl_sync(FULL, target, lead);
+      st0 = __shfl_sync(FULL, st0, lead);
+      const unsigned long long old_tag = __shfl_sync(FULL, other, lead);
+      const uint32_t latest = __shfl_sync(FULL, (second >> slot) & 1u, lead);
+      // rank 0 replaces the other version, rank 1 the latest, rank 2 rank 0's, ...
+      const uint32_t my_slot = (rank & 1u) ? latest : 1u - latest;
+      const bool inst = cand_me && rank + 2u >= n_group;
+      const bool early = inst && my_slot != latest;
+      unsigned long long* my_tag = p.tag + (size_t)target * D + my_slot;
+      constexpr unsigned long long kNoTag = (unsigned long long)kEmptyTs << 32;
+      if (early) st_relaxed_gpu(my_tag, kNoTag);  // readers: moving
+      fence_acq_rel_gpu();
       bool ok_wait = true;
       if (lane == 0)
-        ok_wait = bounded_wait([&] { return ld_acquire_cta(&ms.rep) == seq; }, &p.gs->error,
-                               ERR_WAIT_REPLY, p.spin_log2);
-      ok_wait = __shfl_sync(0xFFFFFFFFu, ok_wait, 0);
+        ok_wait = bounded_wait_fast([&] { return ld_acquire_cta(&ms.rep) == seq; }, &p.gs->error,
+                                    ERR_WAIT_REPLY, p.spin_log2);
+      ok_wait = __shfl_sync(FULL, ok_wait, 0);
       if (!ok_wait) {
+        if (early) st_relaxed_gpu(my_tag, old_tag);
         failed = true;
         break;
       }
       (void)ld_acquire_cta(&ms.rep);
       const uint32_t base = ms.base;
       const uint32_t my_ts = base + 1 + __popc(cand & lanemask_lt());
-      fence_acq_rel_gpu();
-      if (cand_me) st_relaxed_gpu(owner_word(p.cw, target), kPendingFlag | my_ts);
-      bool valid = cand_me;
-      if (cand_me) {
+      // the group's first timestamp in its lock (no timestamp of another SET of this cache set
+      // lies between the group's), then the leader's validation
+      bool valid = cand_me && leader;
+      if (valid) {
+        st_relaxed_gpu(&p.cw[target], ((unsigned long long)(kPendingFlag | my_ts) << 32) | st0);
         unsigned long long wd[kWays];
 #pragma unroll
         for (int wy = 0; wy < kWays; wy++) wd[wy] = ld_relaxed_gpu(&p.cw[e0 + wy]);
 #pragma unroll
         for (int wy = 0; wy < kWays; wy++) {
-          if (!valid) continue;
+          if (!valid || wy == slot) continue;  // (the target's stamp is held)
           // a lock of an earlier or not yet numbered holder: wait (bounded) for its outcome;
           // a later holder is ordered after this SET and is ignored
           bool settled = false;
@@ -380,8 +427,33 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
           valid = settled && (uint32_t)wd[wy] == stw[wy];
         }
       }
-      const uint32_t okm = __ballot_sync(0xFFFFFFFFu, valid);
-      if (lane == 0) stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(cand & ~okm));
+      valid = __shfl_sync(FULL, valid, lead) && cand_me;
+      const uint32_t okm = __ballot_sync(FULL, valid);
+      if (lane == 0) {
+        stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(cand & ~okm));
+        stat_add(sm.stat, ST_COMMIT_UPDATE, __popc(okm));
+      }
+      if (__any_sync(FULL, valid && inst && !early)) {  // the latest version is replaced too
+        if (valid && inst && !early) st_relaxed_gpu(my_tag, kNoTag);
+        fence_acq_rel_gpu();
+      }
+      if (valid && inst) {
+        uint4* rec = p.rec + ((size_t)target * D + my_slot) * 4;
+        st_relaxed_gpu_v4(rec, make_uint4(tick, 0u, 0u, 0u));
+        st_relaxed_gpu_v4(rec + 1, key);
+        st_relaxed_gpu_v4(rec + 2, nv0);
+        st_relaxed_gpu_v4(rec + 3, nv1);
+      }
+      fence_acq_rel_gpu();
+      if (valid && inst)
+        st_relaxed_gpu(my_tag, ((unsigned long long)my_ts << 32) | th);
+      else if (early)
+        st_relaxed_gpu(my_tag, old_tag);
+      fence_acq_rel_gpu();  // with the relaxed store below, the release of the stamp
+      __syncwarp();
+      const uint32_t last_ts = __shfl_sync(FULL, my_ts, group ? 31u - __clz(group) : lane);
+      if (cand_me && leader)
+        st_relaxed_gpu(&p.cw[target], (unsigned long long)(valid ? last_ts : st0));
       if (p.log && cand_me) {
         const uint32_t li = my_ts - 1 - p.log_base;
         if (li < p.log_cap)
@@ -389,48 +461,14 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
         else
           raise_error(&p.gs->error, ERR_CAPACITY);
       }
-      if (valid) {  // install: an empty version first, else the oldest (we hold the lock)
-        const size_t v0 = (size_t)target * D;
-        int vic = 0;
-        uint32_t vkey = 0xFFFFFFFFu;
-#pragma unroll
-        for (int j = 0; j < D; j++) {
-          const uint32_t k = tag_ts(ld_relaxed_gpu(p.tag + v0 + j)) + 1u;
-          if (j == 0 || k < vkey) {
-            vkey = k;
-            vic = j;
-          }
-        }
-        const size_t v = v0 + vic;
-        st_relaxed_gpu(p.tag + v, (unsigned long long)kEmptyTs << 32);  // readers: moving
-        __threadfence();
-        st_relaxed_gpu_v4(p.rec + v * 4, make_uint4(tick, 0u, 0u, 0u));
-        st_relaxed_gpu_v4(p.rec + v * 4 + 1, key);
-        st_relaxed_gpu_v4(p.rec + v * 4 + 2, nv0);
-        st_relaxed_gpu_v4(p.rec + v * 4 + 3, nv1);
-        __threadfence();
-        st_relaxed_gpu(p.tag + v, ((unsigned long long)my_ts << 32) | th);
+      if (valid) {
         if (p.log) p.outcome[r] = my_ts;
         p.found[r] = 0u;
         p.val_out[2 * r] = make_uint4(0, 0, 0, 0);
         p.val_out[2 * r + 1] = make_uint4(0, 0, 0, 0);
       }
-      __threadfence();  // with the relaxed store below, the release of the stamp
-      if (cand_me) {
-        if (valid)
-          st_relaxed_gpu(&p.cw[target], (unsigned long long)my_ts);
-        else
-          st_relaxed_gpu(owner_word(p.cw, target), 0u);
-      }
       complete_range(p.done, p.done_mask, p.gs, base + 1, base + __popc(cand));
-      if (lane == 0) stat_add(sm.stat, ST_COMMIT_UPDATE, __popc(okm));
       pending &= ~okm;
-      uint32_t err = 0;
-      if (lane == 0) err = ld_relaxed_gpu(&p.gs->error);
-      if (__shfl_sync(0xFFFFFFFFu, err, 0) != 0) {
-        failed = true;
-        break;
-      }
     }
   }
   return !failed;

@@ -84,3 +84,25 @@ def test_mixed_round_is_rejected():
         with pytest.raises(cg.CsmvError) as e:
             cache.run(req)
         assert e.value.status == 1
+
+
+@pytest.mark.parametrize("n_sets", [1, 3, 64])
+@pytest.mark.parametrize("pattern", ["all_one", "pairs", "triples", "alternate", "mostly_one"])
+def test_sets_of_one_key_in_a_round_exact(pattern, n_sets):
+    """Rounds whose SETs repeat keys (they commit together under one lock) and share cache sets with
+    other keys, as inserts, refreshes and evictions, beside GETs of the same keys: one warp, then
+    many, replayed exactly."""
+    rng = np.random.default_rng(n_sets)
+    req = _mixed_requests(5, 32 * 48, 64, 50)
+    lane = np.arange(req.n_req) % 32
+    rnd = np.arange(req.n_req) // 32
+    ids = {"all_one": rnd * 0, "pairs": rnd % 3 * 16 + lane // 2, "triples": lane // 3,
+           "alternate": rnd % 2 * 2 + lane % 2,
+           "mostly_one": np.where(rng.random(req.n_req) < 0.8, 7, rng.integers(0, 64, req.n_req))}[pattern]
+    src = _mixed_requests(5, 32 * 400, 64, 50)  # a request of every key id: its key words
+    first = {int(k): i for i, k in reversed(list(enumerate(src.key[:, 0])))}
+    req.key[:] = src.key[[first[int(i)] for i in ids]]
+    for shape in (dict(client_warps=1, ctas=1), dict(client_warps=4, ctas=8)):
+        with cg.Memcd(n_sets=n_sets, max_req=req.n_req, **shape) as cache:
+            for _ in range(2):
+                memcd_run_checked(cache, req)
