@@ -1,7 +1,7 @@
 // mlp_engine.cu - C-ABI of the conflict predictor's network (include/csmv.h, csmv_mlp_*).
 //
 // Device state per handle: fp32 master parameters, Adam moments and the gradient accumulator
-// (kMlpParams floats each), bf16 copies of W1/W2/w3 for the kernels, one loss word. Every call
+// (kMlpParams floats each), bf16 copies of the weights for the kernels, one loss sum. Every call
 // runs on the handle's stream and returns once that stream is idle.
 #include <cmath>
 #include <cstring>
@@ -18,9 +18,10 @@ static_assert(kMlpIn == CSMV_MLP_IN && kMlpHid == CSMV_MLP_HIDDEN, "network shap
 struct csmv_mlp_t {
   int device = 0, n_sms = 0;
   cudaStream_t stream = nullptr;
-  float *master = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr, *loss = nullptr;
-  __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
-  unsigned char* wimg = nullptr;   // weights and biases as the inference kernel's operands
+  float *master = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
+  double* loss = nullptr;          // summed over the samples of the last gradient
+  __nv_bfloat16 *w2 = nullptr, *w3 = nullptr;
+  unsigned char* wimg = nullptr;   // weights and biases in the layout of the MMAs' operands
   // Host word that the inference kernel writes when a wait of it runs out: this one, where the
   // device reads and writes any host memory (a coherent CPU link), else a mapped allocation
   // (which costs 300 us to make).
@@ -36,7 +37,6 @@ void free_all(csmv_mlp_t* h) {
   cudaFree(h->m);
   cudaFree(h->v);
   cudaFree(h->loss);
-  cudaFree(h->w1);
   cudaFree(h->w2);
   cudaFree(h->w3);
   cudaFree(h->wimg);
@@ -73,7 +73,7 @@ extern "C" csmv_status csmv_mlp_create(int32_t device, uint64_t seed, csmv_mlp_t
     size_t bytes;
   } allocs[] = {{(void**)&h->master, pb}, {(void**)&h->grad, pb}, {(void**)&h->m, pb},
                 {(void**)&h->v, pb}, {(void**)&h->loss, 16},
-                {(void**)&h->w1, kMlpIn * kMlpHid * 2}, {(void**)&h->w2, kMlpHid * kMlpHid * 2},
+                {(void**)&h->w2, kMlpHid * kMlpHid * 2},
                 {(void**)&h->w3, kMlpHid * 2}, {(void**)&h->wimg, kTcImageBytes}};
   for (auto& a : allocs)
     if ((st = cuda_status(cudaMalloc(a.p, a.bytes), "cudaMalloc")) != CSMV_OK) return fail(st);
@@ -94,7 +94,7 @@ extern "C" csmv_status csmv_mlp_create(int32_t device, uint64_t seed, csmv_mlp_t
     return fail(st);
   if ((st = cuda_status(cudaFuncSetAttribute((const void*)mlp_grad_kernel,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(MlpSmem)),
+                                             (int)sizeof(MlpGradSmem)),
                         "cudaFuncSetAttribute")) != CSMV_OK ||
       (st = cuda_status(cudaFuncSetAttribute((const void*)mlp_forward_tc_kernel,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -127,7 +127,7 @@ extern "C" csmv_status csmv_mlp_set_params(csmv_mlp_t* h, const float* host_para
   CSMV_CUDA(cudaMemsetAsync(h->m, 0, pb, h->stream));
   CSMV_CUDA(cudaMemsetAsync(h->v, 0, pb, h->stream));
   CSMV_CUDA(cudaMemsetAsync(h->wimg, 0, kTcImageBytes, h->stream));
-  mlp_round_weights_kernel<<<32, 256, 0, h->stream>>>(h->master, h->w1, h->w2, h->w3, h->wimg);
+  mlp_round_weights_kernel<<<(kMlpParams + 255) / 256, 256, 0, h->stream>>>(h->master, h->w2, h->w3, h->wimg);
   CSMV_CUDA(cudaGetLastError());
   CSMV_CUDA(cudaStreamSynchronize(h->stream));
   h->steps = 0;
@@ -165,9 +165,9 @@ csmv_status csmv_mlp_launch_grad(csmv_mlp_t* h, uint32_t n, const void* dev_x, c
   if (n == 0) return CSMV_OK;
   const uint32_t tiles = (n + kMlpTile - 1) / kMlpTile;
   const uint32_t grid = tiles < (uint32_t)h->n_sms ? tiles : (uint32_t)h->n_sms;
-  CSMV_CUDA(cudaMemsetAsync(h->loss, 0, 4, stream));
-  mlp_grad_kernel<<<grid, kMlpThreads, sizeof(MlpSmem), stream>>>(
-      static_cast<const __nv_bfloat16*>(dev_x), dev_y, n, h->w1, h->w2, h->w3, h->master, h->grad,
+  CSMV_CUDA(cudaMemsetAsync(h->loss, 0, 8, stream));
+  mlp_grad_kernel<<<grid, kMlpThreads, sizeof(MlpGradSmem), stream>>>(
+      static_cast<const __nv_bfloat16*>(dev_x), dev_y, n, h->wimg, h->w2, h->w3, h->master, h->grad,
       h->loss);
   return cuda_status(cudaGetLastError(), "mlp_grad_kernel");
 }
@@ -175,12 +175,12 @@ csmv_status csmv_mlp_launch_grad(csmv_mlp_t* h, uint32_t n, const void* dev_x, c
 csmv_status csmv_mlp_launch_adam(csmv_mlp_t* h, float lr, cudaStream_t stream) {
   h->steps++;
   const float b1t = (float)std::pow(0.9, (double)h->steps), b2t = (float)std::pow(0.999, (double)h->steps);
-  mlp_adam_kernel<<<32, 256, 0, stream>>>(h->master, h->grad, h->m, h->v, lr, b1t, b2t, h->w1,
-                                          h->w2, h->w3, h->wimg);
+  mlp_adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, stream>>>(h->master, h->grad, h->m, h->v, lr, b1t, b2t, h->w2,
+                                          h->w3, h->wimg);
   return cuda_status(cudaGetLastError(), "mlp_adam_kernel");
 }
 
-float* csmv_mlp_loss_ptr(csmv_mlp_t* h) { return h->loss; }
+double* csmv_mlp_loss_ptr(csmv_mlp_t* h) { return h->loss; }
 
 // After the stream of a forward launch is idle: did one of its bounded waits run out?
 csmv_status csmv_mlp_forward_status(csmv_mlp_t* h) {
@@ -206,10 +206,10 @@ extern "C" csmv_status csmv_mlp_grad(csmv_mlp_t* h, uint32_t n, const uint16_t* 
   CSMV_CUDA(cudaSetDevice(h->device));
   csmv_status st = csmv_mlp_launch_grad(h, n, dev_x, dev_y, h->stream);
   if (st != CSMV_OK) return st;
-  float l = 0.f;
-  CSMV_CUDA(cudaMemcpyAsync(&l, h->loss, 4, cudaMemcpyDeviceToHost, h->stream));
+  double l = 0.0;
+  CSMV_CUDA(cudaMemcpyAsync(&l, h->loss, 8, cudaMemcpyDeviceToHost, h->stream));
   CSMV_CUDA(cudaStreamSynchronize(h->stream));
-  if (host_loss) *host_loss = l / (float)n;
+  if (host_loss) *host_loss = (float)(l / (double)n);
   return CSMV_OK;
 }
 

@@ -25,7 +25,7 @@ csmv_status csmv_mlp_launch_forward(csmv_mlp_t* h, uint32_t n, const void* dev_x
 csmv_status csmv_mlp_launch_grad(csmv_mlp_t* h, uint32_t n, const void* dev_x, const float* dev_y,
                                  cudaStream_t stream);
 csmv_status csmv_mlp_launch_adam(csmv_mlp_t* h, float lr, cudaStream_t stream);
-float* csmv_mlp_loss_ptr(csmv_mlp_t* h);
+double* csmv_mlp_loss_ptr(csmv_mlp_t* h);
 csmv_status csmv_mlp_forward_status(csmv_mlp_t* h);
 
 struct csmv_sched_t {
@@ -237,10 +237,10 @@ extern "C" csmv_status csmv_sched_probe(csmv_sched_t* s, csmv_bank_t* bank,
   SCHED_LAUNCH_CHECK("labels");
   sched_rates_kernel<<<1, kRateBins, 0, s->stream>>>(s->bin_stats, s->rates);
   SCHED_LAUNCH_CHECK("rates");
-  float loss = 0.f;
+  double loss = 0.0;
   for (uint32_t k = 0; k < s->cfg.train_steps; k++) {
     if ((st = csmv_mlp_launch_grad(s->mlp, np, s->x, s->y, s->stream)) != CSMV_OK) return st;
-    if (k == 0) CSMV_CUDA(cudaMemcpyAsync(&loss, csmv_mlp_loss_ptr(s->mlp), 4, cudaMemcpyDeviceToHost, s->stream));
+    if (k == 0) CSMV_CUDA(cudaMemcpyAsync(&loss, csmv_mlp_loss_ptr(s->mlp), 8, cudaMemcpyDeviceToHost, s->stream));
     if ((st = csmv_mlp_launch_adam(s->mlp, s->cfg.lr, s->stream)) != CSMV_OK) return st;
   }
   CSMV_CUDA(cudaEventRecord(s->ev[1], s->stream));
@@ -249,7 +249,7 @@ extern "C" csmv_status csmv_sched_probe(csmv_sched_t* s, csmv_bank_t* bank,
     float ms = 0.f;
     CSMV_CUDA(cudaEventElapsedTime(&ms, s->ev[0], s->ev[1]));
     rep->train_ms = ms;
-    rep->loss = s->cfg.train_steps ? loss / (float)np : 0.f;
+    rep->loss = s->cfg.train_steps ? (float)(loss / (double)np) : 0.f;
     rep->n_probe = np;
   }
   return CSMV_OK;

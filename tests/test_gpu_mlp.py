@@ -142,3 +142,25 @@ def test_forward_after_training_uses_the_new_weights():
             m.adam_step(1e-2)
         m.forward(700, dx.data_ptr(), dp.data_ptr())
         np.testing.assert_allclose(dp.cpu().numpy(), mo.forward(m.params(), x)[0], rtol=0, atol=2e-5)
+
+
+@pytest.mark.parametrize("n,offset", [(15, 0), (64, 1), (65, 3), (152 * 64, 0), (152 * 64 + 1, 8),
+                                      (3 * 152 * 64 + 113, 5)])
+def test_gradient_at_tile_and_grid_edges(n, offset):
+    """The gradient over partial and whole tiles of 64, one to several tiles a CTA, with the
+    features at any element of an allocation (offset elements of 2 bytes): the bounds above, and
+    the second call adds to the first one's."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    x, xb = _features(rng, n)
+    y = (rng.random(n) < 0.4).astype(np.float32)
+    with cg.Mlp(seed=13) as m:
+        params = m.params()
+        whole = torch.full((offset + n * mo.IN,), 0x7FC0, dtype=torch.int16, device="cuda")
+        whole[offset:] = _dev(torch, xb).flatten()
+        dy = _dev(torch, y)
+        losses = [m.grad(n, whole.data_ptr() + 2 * offset, dy.data_ptr()) for _ in range(2)]
+        g = m.grads().astype(np.float64) / 2
+    loss_ref, g_ref = mo.loss_and_grads(params, x, y)
+    assert max(abs(l - loss_ref) for l in losses) < 1e-4 * max(1.0, abs(loss_ref))
+    np.testing.assert_allclose(g, g_ref, rtol=0, atol=1e-4 * np.abs(g_ref).max())
