@@ -15,16 +15,16 @@
 //              takes the account's latest committed version, looked up here
 //   tails      the last write of each account, where its installs start
 // Execution (one CTA, flow_exec_kernel): warp w runs the blocks of 32 consecutive transactions
-//   w, w + 32, w + 64, ...; each lane polls its reads' producers' outputs until all have
+//   w, w + W, w + 2W, ...; each lane polls its reads' producers' outputs until all have
 //   arrived, runs its transfer and publishes the value of each account it writes - new, or
 //   unchanged when the funds were short - to a shared-memory ring (the chain hand-offs) and to
 //   global memory. A transaction waits only on earlier ones and the earliest unfinished one has
 //   all its inputs, so the lane always makes progress; the polls are bounded all the same
-//   (ERR_WAIT_FLOW).
+//   (ERR_WAIT_FLOW). Read-only blocks are passed over.
 // Commit (all SMs):
 //   ranks      exclusive scan of the has-write flags: the writers take consecutive timestamps in
 //              stream order, as in the serial lane
-//   finalize   outcome, commit log and result of every transaction
+//   finalize   outcome, commit log and result of every transaction (read-only sums here)
 //   install    per written account, from its tail back along the producer chain: the last
 //              `depth` actual writes go to the slots the serial lane gives them (writer r of the
 //              run takes the (r mod depth)-th victim of the slots as the run found them: empty
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(256) flow_src_kernel(FlowParams f, const uint3
 }
 
 // ---------------------------------------------------------------------------------------------
-// Execution: one CTA of kFlowExecThreads threads (32 warps).
+// Execution: one CTA.
 //
 // Outputs go to a ring in shared memory (the hand-offs of a dependency chain take a shared-memory
 // round trip) and to `out` in global memory (read by consumers far behind their producer and by
@@ -344,62 +344,47 @@ struct FlowSmem {
   uint32_t failed;
 };
 
-__device__ __forceinline__ unsigned long long ld_relaxed_cta_shared(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.cta.shared.u64 %0, [%1];"
-               : "=l"(v)
-               : "r"((uint32_t)__cvta_generic_to_shared(p))
-               : "memory");
-  return v;
+// A ring word into w, where it is wanted (predicated, so that a warp's other lanes cost nothing).
+__device__ __forceinline__ void ring_load(unsigned long long& w, uint32_t addr, bool wanted) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.relaxed.cta.shared.u64 %0, [%1];\n}"
+      : "+l"(w)
+      : "r"(addr), "r"((uint32_t)wanted)
+      : "memory");
 }
-__device__ __forceinline__ void st_relaxed_cta_shared(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.cta.shared.u64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)),
-               "l"(v)
-               : "memory");
-}
-
-// Value of a read with source word s, for a consumer in block c; false while it has not arrived.
-__device__ __forceinline__ bool flow_fetch(const FlowParams& f, FlowSmem& S, unsigned long long s,
-                                           uint32_t c, unsigned long long tag, uint32_t& x) {
-  if (s & kFlowValue) {
-    x = (uint32_t)s;
-    return true;
-  }
-  const uint32_t j = (uint32_t)s >> 1;
-  if (c - (j >> 5) < kFlowGate) {
-    const unsigned long long wv = ld_relaxed_cta_shared(&S.ring[(uint32_t)s & (2u * kFlowRing - 1u)]);
-    x = (uint32_t)wv;
-    return (uint32_t)(wv >> 32) == j + 1u;
-  }
-  const unsigned long long wv = ld_relaxed_cta_global(&f.out[s]);
-  x = (uint32_t)wv;
-  return (wv & 0xFFFFFFFF00000000ull) == tag;
+__device__ __forceinline__ void ring_store2(uint32_t addr, unsigned long long w0, unsigned long long w1,
+                                            bool wanted) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.relaxed.cta.shared.v2.u64 [%0], {%1, %2};\n}" ::"r"(addr),
+      "l"(w0), "l"(w1), "r"((uint32_t)wanted)
+      : "memory");
 }
 
-// Entry k (< NR) of a lane's register array, without local memory.
-template <uint32_t NR, class T>
-__device__ __forceinline__ T pick(const T (&a)[NR], uint32_t k) {
-  T s = a[0];
-#pragma unroll
-  for (uint32_t q = 1; q < NR; q++) s = k == q ? a[q] : s;
-  return s;
-}
-
-// A transfer's static inputs (producers, committed values, written accounts, divisor) are read
-// at the start of its block, and so are the outputs of producers at least G blocks older (they
-// have finished); the amount is worked out as soon as its extra reads are in. What is left are
-// producers in the ring, with their ring word and tag worked out once: a pass loads all of them
-// at once (independent shared-memory loads) and takes them when all have arrived - a ring word
-// keeps its producer's value until the consumer's block is done. A finished transfer publishes
-// to the ring at once and leaves its global outputs, flags and counts for the end of the block:
-// the passes that carry the dependency chain stay short.
+// Read-only rounds are left to flow_finalize_kernel: nothing waits on them, and when the last
+// transfer is done every output they sum is in memory. (Run here, their 32 reads a lane from
+// memory held up the later blocks of their warp: 12.5 ms instead of 7.9 for 8192 rounds, a fifth
+// of them read-only.)
+//
+// A block's inputs come in ahead of it, a stage a block: op and offsets; then producers and
+// written accounts; then the outputs of producers at least G blocks older than it. A lane holds
+// every read as a word, tag << 32 | value, beside the tag it waits for: a committed value and an
+// old output have it from the start, a producer in the ring gives it one day. A pass loads the
+// words that still lack their tag, works the transfer out for every lane and publishes those
+// whose words are complete - straight-line code, since the chain of hand-offs is as long as its
+// passes are, and the loads of the lanes that wait are all it asks of shared memory. Global
+// outputs, flags and counts are left to the end of the block.
+//
+// Bound by that chain: 8192 rounds of Zipf(0.99) transfers of 4 accounts of 2^20 (the longest
+// chain of hand-offs is 25 K) take 2.65 ms, 106 ns a hand-off, with 8 warps; 7.5 ms when a pass
+// branched on what each lane waited for. 4 warps take 4.3 ms, 6 3.1, 16 3.0 (fewer do not hide the
+// loads at a block's start, more take the chain's warp its issue slots).
 template <uint32_t NR>
 __global__ void __launch_bounds__(kFlowExecThreads, 1) flow_exec_kernel(FlowParams f) {
   extern __shared__ __align__(16) unsigned char flow_smem_raw[];
   FlowSmem& S = *reinterpret_cast<FlowSmem*>(flow_smem_raw);
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const uint32_t nb = f.n_txn / 32u;
-  const unsigned long long tag = (unsigned long long)f.epoch << 32;
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(S.ring);
   uint32_t* err = &f.b.gs->error;
   const uint32_t limit = 1u << f.b.spin_log2;  // spin_log2 <= 30
   for (uint32_t k = threadIdx.x; k < 2u * kFlowRing; k += blockDim.x) S.ring[k] = 0ull;
@@ -421,30 +406,57 @@ __global__ void __launch_bounds__(kFlowExecThreads, 1) flow_exec_kernel(FlowPara
     return true;
   };  // (called with it = 255, 511, ... by the execution loop: limit >= 1024)
   uint32_t finished = 0;  // this warp's blocks
-  uint32_t op_n = 0, e0_n = 0;  // the next block's op and element offset, loaded ahead
-  if (w < nb) {
-    op_n = f.b.op[w * 32u + lane];
-    e0_n = f.eoff[w * 32u + lane];
-  }
+  const uint32_t step = 32u * nw;
+  struct Head {  // op and offsets of a lane's transaction
+    uint32_t op, e0, off;
+  };
+  struct Body {  // its producers and accounts, and what is there of their outputs
+    uint32_t op, a0, a1;
+    unsigned long long sv[NR];
+  };
+  auto head = [&](uint32_t i, Head& h) {
+    if (i >= f.n_txn) return;
+    h.op = f.b.op[i];
+    h.e0 = f.eoff[i];
+    h.off = f.b.off[i];
+  };
+  auto body = [&](uint32_t i, const Head& h, Body& d) {
+    d.op = h.op;
+    if (i >= f.n_txn || CSMV_OP_KIND(h.op) == CSMV_KIND_READONLY) return;
+#pragma unroll
+    for (uint32_t k = 0; k < NR; k++) d.sv[k] = k < CSMV_OP_NREADS(h.op) ? __ldg(&f.src[h.e0 + k]) : kFlowValue;
+    d.a0 = f.b.addr[h.off];
+    d.a1 = f.b.addr[h.off + 1];
+  };
+  // read k's word is in global memory (its producer is G blocks older at least)
+  auto is_old = [&](unsigned long long s, uint32_t b) {
+    return !(s & kFlowValue) && b - ((uint32_t)s >> 6) >= kFlowGate;
+  };
+  auto outputs = [&](uint32_t i, const Body& d, unsigned long long (&gv)[NR]) {
+    if (i >= f.n_txn || CSMV_OP_KIND(d.op) == CSMV_KIND_READONLY) return;
+#pragma unroll
+    for (uint32_t k = 0; k < NR; k++)
+      if (is_old(d.sv[k], i >> 5)) gv[k] = ld_relaxed_cta_global(&f.out[d.sv[k]]);
+  };
+  Head h2{};
+  Body d1{}, d0;
+  unsigned long long g0[NR] = {};
+  const uint32_t i0 = w * 32u + lane;
+  head(i0, h2);
+  body(i0, h2, d1);
+  head(i0 + step, h2);
+  outputs(i0, d1, g0);
   for (uint32_t b = w; b < nb; b += nw) {
     const uint32_t i = b * 32u + lane;
-    const uint32_t op = op_n, e0 = e0_n;
-    if (b + nw < nb) {
-      op_n = f.b.op[i + 32u * nw];
-      e0_n = f.eoff[i + 32u * nw];
-    }
-    const uint32_t nr = CSMV_OP_NREADS(op);
-    const bool ro = CSMV_OP_KIND(op) == CSMV_KIND_READONLY;
-    unsigned long long sv[NR];
-    uint32_t a0 = 0, a1 = 0;
-    if (!ro) {
-      const uint32_t off = f.b.off[i];
+    unsigned long long wv[NR];
 #pragma unroll
-      for (uint32_t k = 0; k < NR; k++) sv[k] = k < nr ? __ldg(&f.src[e0 + k]) : kFlowValue;
-      a0 = f.b.addr[off];
-      a1 = f.b.addr[off + 1];
-    }
-    if (b >= kFlowGate) {  // every block <= b - G finished
+    for (uint32_t k = 0; k < NR; k++) wv[k] = g0[k];
+    d0 = d1;
+    body(i + step, h2, d1);
+    head(i + 2u * step, h2);
+    const uint32_t op = d0.op;
+    const bool ro = CSMV_OP_KIND(op) == CSMV_KIND_READONLY;  // of the whole block
+    if (!ro && b >= kFlowGate) {  // every block <= b - G finished
       const uint32_t q = b - kFlowGate;
       for (uint32_t it = 0;; ++it) {
         bool ok = true;
@@ -454,120 +466,75 @@ __global__ void __launch_bounds__(kFlowExecThreads, 1) flow_exec_kernel(FlowPara
       }
       __syncwarp();
     }
-    int32_t v0 = 0, v1 = 0;
-    uint32_t acc = 0;  // extra reads of a transfer; every read past the first two of a scan
-    uint32_t pm = 0;   // a transfer's reads waiting on the ring
-    unsigned long long gpend = 0;  // reads waiting on global memory (a scan: all of them)
-    auto take = [&](uint32_t k, uint32_t x) {
-      v0 = k == 0 ? (int32_t)x : v0;
-      v1 = k == 1 ? (int32_t)x : v1;
-      acc += k >= 2 ? x : 0u;
-    };
-    const ModMagic mm(ro ? 1u : CSMV_OP_AMOD(op));
-    uint32_t ridx[NR], rtag[NR];
-    if (!ro) {
-      // committed values, and outputs of producers that finished (all loads issued together)
-      unsigned long long gv[NR];
-#pragma unroll
-      for (uint32_t k = 0; k < NR; k++) {
-        const unsigned long long s = sv[k];
-        gv[k] = s;
-        if (k < nr && !(s & kFlowValue) && b - ((uint32_t)s >> 6) >= kFlowGate)
-          gv[k] = ld_relaxed_cta_global(&f.out[s]);
-        ridx[k] = (uint32_t)s & (2u * kFlowRing - 1u);
-        rtag[k] = ((uint32_t)s >> 1) + 1u;
-      }
-#pragma unroll
-      for (uint32_t k = 0; k < NR; k++) {
-        if (k >= nr) continue;
-        const unsigned long long s = sv[k];
-        if (s & kFlowValue) {
-          take(k, (uint32_t)s);
-        } else if (b - ((uint32_t)s >> 6) >= kFlowGate) {
-          if ((gv[k] & 0xFFFFFFFF00000000ull) == tag)
-            take(k, (uint32_t)gv[k]);
-          else
-            gpend |= 1ull << k;
-        } else {
-          pm |= 1u << k;
-        }
-      }
-    } else {
-      gpend = (1ull << nr) - 1ull;  // a scan: every read through flow_fetch (nr <= 63)
-    }
-    // the amount, as soon as every extra read is in (usually here, before any wait)
-    uint32_t amt = 0;
-    bool amt_known = false;
-    auto try_amount = [&]() {
-      if (!ro && !amt_known && ((pm | (uint32_t)gpend) & ~3u) == 0u) {
-        amt = 1u + mm.mod(CSMV_OP_AMT0(op) - 1u + acc);
-        amt_known = true;
-      }
-    };
-    try_amount();
-    bool done = false, hw = false;
-    uint32_t o0 = 0, o1 = 0;
-    for (uint32_t it = 0;; ++it) {
-      if (!done) {
-        if (pm) {  // every ring read polled at once; all are taken when all have arrived
-          uint32_t rdy = 0, xv[NR];
-#pragma unroll
-          for (uint32_t k = 0; k < NR; k++) {
-            xv[k] = 0u;
-            if ((pm >> k) & 1u) {
-              const unsigned long long wv = ld_relaxed_cta_shared(&S.ring[ridx[k]]);
-              xv[k] = (uint32_t)wv;
-              rdy |= (uint32_t)((uint32_t)(wv >> 32) == rtag[k]) << k;
-            }
-          }
-          if (rdy == pm) {
-#pragma unroll
-            for (uint32_t k = 0; k < NR; k++)
-              if ((pm >> k) & 1u) take(k, xv[k]);
-            pm = 0u;
-          }
-        }
-        if (gpend) {
-          for (unsigned long long m = gpend; m; m &= m - 1ull) {
-            const uint32_t k = (uint32_t)__ffsll((long long)m) - 1u;
-            uint32_t x;
-            if (flow_fetch(f, S, ro ? __ldg(&f.src[e0 + k]) : pick<NR>(sv, k), b, tag, x)) {
-              take(k, x);
-              gpend &= ~(1ull << k);
-            }
-          }
-        }
-        if (pm == 0u && gpend == 0ull) {
-          done = true;
-          if (!ro) {
-            try_amount();
-            hw = CSMV_OP_KIND(op) == CSMV_KIND_TRANSFER_ALWAYS || v0 >= (int32_t)amt;
-            o0 = hw ? (uint32_t)v0 - amt : (uint32_t)v0;
-            o1 = hw ? (uint32_t)v1 + amt : (uint32_t)v1;
-            const unsigned long long rt = (unsigned long long)(i + 1u) << 32;
-            const uint32_t r0 = (2u * i) & (2u * kFlowRing - 1u);
-            if (a0 != a1) st_relaxed_cta_shared(&S.ring[r0], rt | o0);
-            st_relaxed_cta_shared(&S.ring[r0 + 1u], rt | o1);
-          }
-        } else {
-          try_amount();
-        }
-      }
-      if (__all_sync(0xFFFFFFFFu, done)) break;
-      // (no warp barrier between passes: a ring word read before its store is only "not yet")
-      if ((it & 255u) == 255u && !keep_polling(it)) return;
-    }
-    // off the chain: global outputs, flags, counts, scan results
     if (ro) {
-      if (f.b.log) f.b.result[i] = (int32_t)((uint32_t)v0 + (uint32_t)v1 + acc);
+      outputs(i + step, d1, g0);
       f.wflag[i] = 0u;
     } else {
-      if (a0 != a1) st_relaxed_cta_global(&f.out[2u * i], tag | o0);
-      st_relaxed_cta_global(&f.out[2u * i + 1u], tag | o1);
+      uint32_t addr[NR], tag[NR];
+#pragma unroll
+      for (uint32_t k = 0; k < NR; k++) {
+        const unsigned long long s = d0.sv[k];
+        addr[k] = ring + 8u * ((uint32_t)s & (2u * kFlowRing - 1u));
+        if (s & kFlowValue) {
+          tag[k] = 0u;
+          wv[k] = (uint32_t)s;
+        } else if (is_old(s, b)) {
+          tag[k] = f.epoch;
+          // not there when it was loaded ahead; its producer has finished by now
+          for (uint32_t it = 0; (uint32_t)(wv[k] >> 32) != f.epoch; ++it) {
+            wv[k] = ld_relaxed_cta_global(&f.out[s]);
+            if (it >= limit) {
+              raise_error(err, ERR_WAIT_FLOW);
+              break;
+            }
+          }
+        } else {
+          tag[k] = ((uint32_t)s >> 1) + 1u;
+          wv[k] = 0ull;
+        }
+      }
+      __syncwarp();
+      const ModMagic mm(CSMV_OP_AMOD(op));
+      const bool always = CSMV_OP_KIND(op) == CSMV_KIND_TRANSFER_ALWAYS;
+      const uint32_t amt0 = CSMV_OP_AMT0(op) - 1u;
+      const uint32_t mine = ring + 8u * ((2u * i) & (2u * kFlowRing - 1u));
+      const unsigned long long rt = (unsigned long long)(i + 1u) << 32;
+      bool done = false, hw = false;
+      uint32_t o0 = 0, o1 = 0;
+      auto pass = [&]() {
+        bool ready = !done;
+        uint32_t acc = amt0;
+#pragma unroll
+        for (uint32_t k = 0; k < NR; k++) ring_load(wv[k], addr[k], (uint32_t)(wv[k] >> 32) != tag[k]);
+#pragma unroll
+        for (uint32_t k = 0; k < NR; k++) {
+          ready &= (uint32_t)(wv[k] >> 32) == tag[k];
+          if (k >= 2) acc += (uint32_t)wv[k];
+        }
+        const uint32_t v0 = (uint32_t)wv[0], v1 = (uint32_t)wv[1], amt = 1u + mm.mod(acc);
+        hw = always || (int32_t)v0 >= (int32_t)amt;
+        o0 = hw ? v0 - amt : v0;
+        o1 = hw ? v1 + amt : v1;
+        // (a lane with one account has it in slot 1; no one reads its slot 0)
+        ring_store2(mine, rt | o0, rt | o1, ready);
+        done |= ready;
+      };
+      for (uint32_t it = 0;; ++it) {
+        pass();
+        pass();
+        if (__all_sync(0xFFFFFFFFu, done)) break;
+        // (no warp barrier between passes: a ring word read before its store is only "not yet")
+        if ((it & 255u) == 255u && !keep_polling(it)) return;
+      }
+      outputs(i + step, d1, g0);
+      // off the chain: global outputs, flags, counts
+      const unsigned long long et = (unsigned long long)f.epoch << 32;
+      if (d0.a0 != d0.a1) st_relaxed_cta_global(&f.out[2u * i], et | o0);
+      st_relaxed_cta_global(&f.out[2u * i + 1u], et | o1);
       f.wflag[i] = hw ? 1u : 0u;
       if (hw) {
-        atomicAdd(&f.cnt[a0], 1u);
-        if (a1 != a0) atomicAdd(&f.cnt[a1], 1u);
+        atomicAdd(&f.cnt[d0.a0], 1u);
+        if (d0.a1 != d0.a0) atomicAdd(&f.cnt[d0.a1], 1u);
       }
     }
     __syncwarp();  // every lane's outputs before the block is announced
@@ -595,7 +562,19 @@ __global__ void __launch_bounds__(256) flow_finalize_kernel(FlowParams f) {
     } else {
       f.b.outcome[i] = (base0 + r) | kSnapFlag;  // after every earlier writer
     }
-    if (CSMV_OP_KIND(f.b.op[i]) != CSMV_KIND_READONLY) f.b.result[i] = 0;
+    int32_t sum = 0;
+    const uint32_t op = f.b.op[i];
+    if (CSMV_OP_KIND(op) == CSMV_KIND_READONLY) {  // its producers' outputs are all there
+      const uint32_t nr = CSMV_OP_NREADS(op), e0 = f.eoff[i];
+      uint32_t acc = 0;
+#pragma unroll 8
+      for (uint32_t k = 0; k < nr; k++) {
+        const unsigned long long sv = f.src[e0 + k];
+        acc += (uint32_t)(sv & kFlowValue ? sv : f.out[sv]);
+      }
+      sum = (int32_t)acc;
+    }
+    f.b.result[i] = sum;
   }
   if (f.b.txn_aborts) f.b.txn_aborts[i] = 0u;
 }

@@ -366,6 +366,33 @@ def test_flow_lane_equals_serial_lane(case):
         assert err is None, err
 
 
+@pytest.mark.parametrize("up,ro,warps", [(2, 0, 1), (3, 40, 3), (4, 20, 8), (8, 10, 5), (8, 90, 16)])
+def test_flow_lane_old_and_recent_producers(up, ro, warps):
+    """Reads whose producers are in the lane's window (128 blocks), at its edge and far behind it,
+    read-only blocks among them, streams that no number of warps divides: balances and sums of
+    the serial oracle."""
+    torch = pytest.importorskip("torch")
+    n_acc, n = 3000, 32 * 389
+    w = c1_workload(n_txn=n, n_accounts=n_acc, dist=cg.DIST_UNIFORM, up_reads=up, pr_read_pct=ro,
+                    seed=up + ro)
+    s = cg.generate(w)
+    hot = np.flatnonzero((s.op & 3) != 0)[::64]  # every other round writes account 0 once
+    for t in hot:
+        if 0 not in s.addr[s.off[t]:s.off[t] + up]:
+            s.addr[s.off[t]] = 0
+    ds, keep = to_device(torch, s)
+    with cg.Bank(n_accounts=n_acc, max_txn=n, version_depth=4, flow_warps=warps) as bank:
+        bank.load()
+        st = bank.run_flow_device(ds)
+        log_txn, outcome, result = bank.log(n, st.final_ts)
+        slots, vals = bank.versions(), bank.values()
+    init = np.full(n_acc, 1000, np.int32)
+    err = orc.check(s.op, s.off, s.addr, n_acc, init, 4, st.final_ts, log_txn, outcome, result,
+                    slots)
+    assert err is None, err
+    np.testing.assert_array_equal(vals, orc.serial(s.op, s.off, s.addr, n_acc, init)[0])
+
+
 def test_flow_lane_interleaves_with_engine_and_serial_lane():
     """Concurrent run, dataflow run, serial-lane run, dataflow run on one bank: the commit order
     carries across them and the concatenated log replays exactly."""
