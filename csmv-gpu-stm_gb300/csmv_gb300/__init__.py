@@ -463,7 +463,7 @@ class Bank:
         return st
 
     def run_serial_device(self, dev_stream: BankStream) -> Stats:
-        """The serial lane: stream order, one warp, exclusive (csmv_bank_run_serial_device)."""
+        """The serial lane: stream order, exclusive (csmv_bank_run_serial_device)."""
         st = Stats()
         rc = lib().csmv_bank_run_serial_device(self._h, C.byref(dev_stream), C.byref(st))
         self.last_stats = st

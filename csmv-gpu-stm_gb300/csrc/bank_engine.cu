@@ -504,6 +504,14 @@ extern "C" csmv_status csmv_bank_run_device(csmv_bank_t* h, const csmv_bank_stre
   return st;
 }
 
+// Serial-lane runs of these sizes go to the dataflow lane, which leaves the same state. Its
+// analysis and commit are some 35 launches, 190-250 us whatever the size; the serial kernel's one
+// warp takes 4.5 (transfers of 2 accounts, uniform) to 14 us a round. At 64 rounds they take
+// 316-893 us and 225-287 us, but a first run also makes the lane's buffers (351 against 386 us for
+// the shortest rounds); at 128 rounds 586-1746 and 245-330, at 1024 of Zipf(0.99) 11.8 ms and
+// 0.7 ms. At the upper end the buffers would be a GB and more.
+constexpr uint32_t kSerialAsFlow = 96 * 32, kFlowSerialMax = 1u << 22;
+
 extern "C" csmv_status csmv_bank_run_serial_device(csmv_bank_t* h, const csmv_bank_stream* s,
                                                    csmv_stats* out) {
   if (!h) return CSMV_ERR_INVALID_ARG;
@@ -519,8 +527,14 @@ extern "C" csmv_status csmv_bank_run_serial_device(csmv_bank_t* h, const csmv_ba
   }
   CSMV_CUDA(cudaSetDevice(h->cfg.device));
   auto t0 = std::chrono::steady_clock::now();
-  st = launch(h, s->op, s->off, s->addr, s->n_txn, s->txn_aborts, 0, 0, nullptr, s->txn_waits,
-              nullptr, out, true);
+  bool ran = false;
+  if (s->n_txn >= kSerialAsFlow && s->n_txn <= kFlowSerialMax) {
+    if (s->txn_waits) CSMV_CUDA(cudaMemsetAsync(s->txn_waits, 0, (size_t)s->n_txn * 4, h->stream));
+    ran = flow_serial_run(h, s, out, &st);
+  }
+  if (!ran)
+    st = launch(h, s->op, s->off, s->addr, s->n_txn, s->txn_aborts, 0, 0, nullptr, s->txn_waits,
+                nullptr, out, true);
   if (out)
     out->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return st;

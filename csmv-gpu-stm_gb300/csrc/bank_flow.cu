@@ -138,13 +138,15 @@ csmv_status scan(uint32_t* data, uint32_t n, uint32_t* agg, cudaStream_t s) {
 
 uint32_t grid_of(uint64_t n, uint32_t block) { return (uint32_t)((n + block - 1) / block); }
 
-// Everything after the checks; the caller ends the run (statistics, status).
-csmv_status flow_launch(csmv_bank_t* h, const csmv_bank_stream* s) {
+// Everything after the checks; the caller ends the run (statistics, status). *ready: every buffer
+// was there and the execution is launched.
+csmv_status flow_launch(csmv_bank_t* h, const csmv_bank_stream* s, uint32_t spin_log2, bool* ready) {
   const uint32_t n = s->n_txn;
   FlowScratch* f = h->flow;
   cudaStream_t st = h->stream;
   FlowParams p{};
   p.b = bank_params(h, s->op, s->off, s->addr, n, s->txn_aborts);
+  p.b.spin_log2 = spin_log2;
   p.n_txn = n;
   p.eoff = f->eoff;
   p.out = f->out;
@@ -203,6 +205,7 @@ csmv_status flow_launch(csmv_bank_t* h, const csmv_bank_stream* s) {
   else
     flow_exec_kernel<8><<<1, 32 * warps, sizeof(FlowSmem), st>>>(p);
   CSMV_CUDA(cudaGetLastError());
+  *ready = true;
   if ((rc = scan<false>(f->wflag, n, f->agg, st)) != CSMV_OK) return rc;
   flow_finalize_kernel<<<grid_of(n, 256), 256, 0, st>>>(p);
   CSMV_CUDA(cudaGetLastError());
@@ -213,7 +216,45 @@ csmv_status flow_launch(csmv_bank_t* h, const csmv_bank_stream* s) {
   return CSMV_OK;
 }
 
+// One run between begin and end; a failed one leaves no per-account counts behind.
+csmv_status flow_run(csmv_bank_t* h, const csmv_bank_stream* s, uint32_t spin_log2, csmv_stats* out,
+                     bool* ready) {
+  *ready = false;
+  csmv_status st = ensure_txn(h, s->n_txn);
+  if (st != CSMV_OK) return st;
+  h->last_grouped = false;  // the lane installs every write
+  if ((st = bank_begin_run(h)) != CSMV_OK) return st;
+  csmv_status lst = flow_launch(h, s, spin_log2, ready);
+  st = bank_end_run(h, s->n_txn, out);  // waits for the stream whatever happened
+  if (lst != CSMV_OK) st = lst;
+  if (st != CSMV_OK) {
+    csmv_status rs = flow_scratch_reset(h->flow, h->stream);
+    if (rs == CSMV_OK) cudaStreamSynchronize(h->stream);
+  }
+  return st;
+}
+
 }  // namespace
+
+// A serial-lane run as a run of this lane. False: the caller's kernel has to do it, and nothing
+// has been applied - no memory for the buffers, too many accesses, a stream with a malformed
+// round (the serial kernel applies the rounds before it), a wait that ran out.
+bool csmv::flow_serial_run(csmv_bank_t* h, const csmv_bank_stream* s, csmv_stats* out, csmv_status* st) {
+  csmv_stats stats{};
+  bool ready = false;
+  // the serial lane has no limit on waits: at least 2^24 passes (seconds) here
+  const uint32_t spin = h->cfg.spin_limit_log2 > 24u ? h->cfg.spin_limit_log2 : 24u;
+  *st = flow_run(h, s, spin, &stats, &ready);
+  if (*st != CSMV_OK && !ready) {
+    cudaGetLastError();  // an allocation that failed is no error of the next launch
+    flow_scratch_free(h->flow);
+    h->flow = nullptr;
+    return false;
+  }
+  if (stats.error == ERR_DATA || stats.error == ERR_WAIT_FLOW) return false;
+  if (out) *out = stats;
+  return true;
+}
 
 extern "C" csmv_status csmv_bank_run_flow_device(csmv_bank_t* h, const csmv_bank_stream* s,
                                                  csmv_stats* out) {
@@ -234,17 +275,8 @@ extern "C" csmv_status csmv_bank_run_flow_device(csmv_bank_t* h, const csmv_bank
   }
   CSMV_CUDA(cudaSetDevice(h->cfg.device));
   auto t0 = std::chrono::steady_clock::now();
-  if ((st = ensure_txn(h, s->n_txn)) != CSMV_OK) return st;
-  h->last_grouped = false;  // the lane installs every write
-  if ((st = bank_begin_run(h)) != CSMV_OK) return st;
-  csmv_status lst = flow_launch(h, s);
-  st = bank_end_run(h, s->n_txn, out);  // waits for the stream whatever happened
-  if (lst != CSMV_OK) st = lst;
-  if (st != CSMV_OK) {
-    // a failed run may leave per-account counts behind
-    csmv_status rs = flow_scratch_reset(h->flow, h->stream);
-    if (rs == CSMV_OK) cudaStreamSynchronize(h->stream);
-  }
+  bool ready;
+  st = flow_run(h, s, h->cfg.spin_limit_log2, out, &ready);
   if (out)
     out->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return st;

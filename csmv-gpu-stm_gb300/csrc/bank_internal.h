@@ -71,5 +71,7 @@ csmv_status bank_begin_run(csmv_bank_t* h);
 // Records the end event, waits for the stream, reads statistics and the commit cursor into
 // *out and advances the handle's log window; maps a device error to a status.
 csmv_status bank_end_run(csmv_bank_t* h, uint32_t n_txn, csmv_stats* out);
+// A checked serial-lane run by the dataflow lane; false: nothing was applied (bank_flow.cu).
+bool flow_serial_run(csmv_bank_t* h, const csmv_bank_stream* s, csmv_stats* out, csmv_status* st);
 
 }  // namespace csmv

@@ -250,12 +250,14 @@ csmv_status csmv_bank_run(csmv_bank_t* h, const csmv_bank_stream* host_stream,
 csmv_status csmv_bank_run_device(csmv_bank_t* h, const csmv_bank_stream* dev_stream,
                                  csmv_stats* out);
 
-/* Serial lane (no counterpart in the reference): one warp runs the device-resident stream in
- * stream order with the GPU to itself - a round's 32 transfers resolve their dependencies as a
- * chain in lane order and commit together, with no locks, timestamp server or validation -
- * continuing the commit order of the handle (stamp protocol only). Meant for transactions a
- * scheduler predicts to conflict; no other run of the handle may be in flight. Every
- * transaction commits; read-only ones see the state after all earlier ones. */
+/* Serial lane (no counterpart in the reference): the device-resident stream in stream order
+ * with the GPU to itself - with no locks, timestamp server or validation - continuing the commit
+ * order of the handle (stamp protocol only). Meant for transactions a scheduler predicts to
+ * conflict; no other run of the handle may be in flight. Every transaction commits; read-only
+ * ones see the state after all earlier ones. Short streams are run by one warp, a round's 32
+ * transfers resolving their dependencies as a chain in lane order; streams of 96 rounds and more
+ * by the dataflow lane's kernels (below, with their device scratch), which leave the same
+ * state - where these cannot take the stream, by the one warp too. */
 csmv_status csmv_bank_run_serial_device(csmv_bank_t* h, const csmv_bank_stream* dev_stream,
                                         csmv_stats* out);
 

@@ -393,6 +393,65 @@ def test_flow_lane_old_and_recent_producers(up, ro, warps):
     np.testing.assert_array_equal(vals, orc.serial(s.op, s.off, s.addr, n_acc, init)[0])
 
 
+SERIAL_CASES = {  # rounds, accounts, reads of a transfer, read-only %, slots, distribution
+    "96-rounds": (96, 512, 4, 20, 4, cg.DIST_ZIPF),
+    "97-rounds-hot": (97, 16, 3, 30, 2, cg.DIST_UNIFORM),
+    "300-rounds-eight-reads": (300, 1 << 14, 8, 10, 8, cg.DIST_ZIPF),
+    "200-rounds-self-transfers": (200, 64, 2, 0, 16, cg.DIST_UNIFORM),
+}
+
+
+@pytest.mark.parametrize("case", list(SERIAL_CASES))
+@pytest.mark.parametrize("bad", [False, True])
+def test_serial_lane_long_runs_equal_short_runs(case, bad):
+    """A serial-lane run long enough for the dataflow kernels leaves what the same stream leaves
+    when it is run in pieces short enough for the one-warp kernel: outcomes, log, results, version
+    slots. With a malformed round near the end, the rounds before it are applied and the call is
+    refused, as the one-warp kernel does; limits on waits do not apply."""
+    torch = pytest.importorskip("torch")
+    rounds, n_acc, up, ro, depth, dist = SERIAL_CASES[case]
+    n = 32 * rounds
+    s = cg.generate(c1_workload(n_txn=n, n_accounts=n_acc, dist=dist, zipf_theta=0.99,
+                                up_reads=up, pr_read_pct=ro, seed=rounds))
+    if "self" in case:
+        t = np.flatnonzero((s.op & 3) != 0)[::3]
+        s.addr[s.off[t] + 1] = s.addr[s.off[t]]
+    stop = rounds
+    if bad:
+        stop = rounds - 5
+        s.addr[s.off[32 * stop + 7]] = n_acc
+    kw = dict(n_accounts=n_acc, max_txn=n, version_depth=depth, spin_limit_log2=10)
+    with cg.Bank(**kw) as bank:
+        bank.load()
+        ds, keep = to_device(torch, s)
+        if bad:
+            with pytest.raises(cg.CsmvError):
+                bank.run_serial_device(ds)
+        else:
+            st = bank.run_serial_device(ds)
+            assert st.commits == n and st.aborts == 0 and st.rounds == st.sections == rounds
+            log, oc, rs = bank.log(n, st.final_ts)
+            assert st.final_ts == st.commits_update
+        long_slots, long_vals = bank.versions(), bank.values()
+    with cg.Bank(**kw) as bank:
+        bank.load()
+        prev, logs, outs, ress = 0, [], [], []
+        for lo in range(0, stop, 90):
+            hi = min(lo + 90, stop)
+            ds, keep = to_device(torch, sub_stream(s, 32 * lo, 32 * hi))
+            st = bank.run_serial_device(ds)
+            a, b, c = bank.log(32 * (hi - lo), st.final_ts - prev)
+            logs.append(np.where(a != 0xFFFFFFFF, a + 32 * lo, a)), outs.append(b), ress.append(c)
+            prev = st.final_ts
+        slots, vals = bank.versions(), bank.values()
+    np.testing.assert_array_equal(long_slots, slots)
+    np.testing.assert_array_equal(long_vals, vals)
+    if not bad:
+        np.testing.assert_array_equal(oc, np.concatenate(outs))
+        np.testing.assert_array_equal(rs, np.concatenate(ress))
+        np.testing.assert_array_equal(log, np.concatenate(logs))
+
+
 def test_flow_lane_interleaves_with_engine_and_serial_lane():
     """Concurrent run, dataflow run, serial-lane run, dataflow run on one bank: the commit order
     carries across them and the concatenated log replays exactly."""
