@@ -292,10 +292,8 @@ extern "C" csmv_status csmv_bank_run_baseline_device(csmv_bank_t* h, const csmv_
   BankParams p = bank_params(h, s->op, s->off, s->addr, s->n_txn, nullptr);
   p.grp = nullptr;
   h->last_grouped = false;
-  CSMV_CUDA(cudaMemsetAsync(&h->gs->section, 0, 4, h->stream));
-  CSMV_CUDA(cudaMemsetAsync(&h->gs->section_serving, 0, 4, h->stream));
   const uint32_t base0 = h->last_final_ts;
-  st = bank_begin_run(h);
+  st = bank_begin_run(h);  // (the commit section's tickets too)
   if (st != CSMV_OK) return st;
   fn<<<h->ctas, h->cfg.client_warps * 32u, 0, h->stream>>>(p);
   CSMV_CUDA(cudaGetLastError());

@@ -17,6 +17,12 @@ KernelFn pick_kernel_r4(uint32_t depth);
 KernelFn pick_cluster_r4(uint32_t depth);
 size_t cta_shared_bytes_r4(uint32_t n_mail);
 
+// Device words that a run resets (from round_next on) and reads back at its end.
+struct RunState {
+  GlobalSync gs;
+  unsigned long long stats[ST_COUNT];
+};
+
 struct FlowScratch;                                        // bank_flow.cu
 void flow_scratch_free(FlowScratch* f);                    // frees the dataflow lane's buffers
 csmv_status flow_scratch_reset(FlowScratch* f, cudaStream_t s);  // zeroes its per-account counts

@@ -393,6 +393,38 @@ def test_flow_lane_old_and_recent_producers(up, ro, warps):
     np.testing.assert_array_equal(vals, orc.serial(s.op, s.off, s.addr, n_acc, init)[0])
 
 
+@pytest.mark.parametrize("prevalidate", [1, 3])
+@pytest.mark.parametrize("rounds", [1, 2, 3, 4, 7, 12, 13])
+def test_streams_of_few_rounds_on_few_warps(rounds, prevalidate):
+    """Streams of fewer rounds than the handle has warps (3 CTAs of 4): every count of CTAs and of
+    warps a CTA that the launch can take; two runs in a row replay exactly."""
+    torch = pytest.importorskip("torch")
+    n_acc, n = 512, 32 * rounds
+    s = cg.generate(c1_workload(n_txn=2 * n, n_accounts=n_acc, up_reads=3, pr_read_pct=20,
+                                seed=rounds))
+    logs, ends, prev = [], [], 0
+    with cg.Bank(n_accounts=n_acc, max_txn=n, ctas=3, client_warps=4,
+                 prevalidate=prevalidate) as bank:
+        bank.load()
+        for i in range(2):
+            st = bank.run(sub_stream(s, i * n, (i + 1) * n))
+            assert st.commits == n
+            lt, oc, rs = bank.log(n, st.final_ts - prev)
+            logs.append((np.where(lt != 0xFFFFFFFF, lt + i * n, lt).astype(np.uint32), oc, rs))
+            if prevalidate == 3:  # a group leaves one version of an account
+                bits = bank.groups(st.final_ts - prev).view(np.uint8)
+                ends.append(np.unpackbits(bits, bitorder="little")[:st.final_ts - prev])
+            prev = st.final_ts
+        slots = bank.versions()
+    groups = None
+    if prevalidate == 3:
+        bits = np.concatenate(ends + [np.zeros(-prev % 32, np.uint8)])
+        groups = np.packbits(bits, bitorder="little").view(np.uint32)
+    err = orc.check(s.op, s.off, s.addr, n_acc, np.full(n_acc, 1000, np.int32), 4, prev,
+                    *[np.concatenate(x) for x in zip(*logs)], slots, groups=groups)
+    assert err is None, err
+
+
 SERIAL_CASES = {  # rounds, accounts, reads of a transfer, read-only %, slots, distribution
     "96-rounds": (96, 512, 4, 20, 4, cg.DIST_ZIPF),
     "97-rounds-hot": (97, 16, 3, 30, 2, cg.DIST_UNIFORM),
