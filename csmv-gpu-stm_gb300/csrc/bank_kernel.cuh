@@ -342,8 +342,9 @@ static __device__ uint32_t complete_prefix(const uint32_t* done, uint32_t done_m
   return n;
 }
 
-// Mark timestamps [lo, hi] (hi - lo < 32) complete (their write-back is visible), then see that the
-// clock moves over the longest complete prefix; warp-collective. A range is published atomically
+// Mark timestamps [lo, hi] (hi - lo < 32) complete (lane 0 has fenced after a warp barrier behind
+// their write-back), then see that the clock moves over the longest complete prefix;
+// warp-collective. A range is published atomically
 // for the clock: of its (at most two) bitmap words the higher is set first, fenced, then the
 // lower, so a scan that sees the range's first bit and reads the next word after it sees all of
 // it - the clock never stops inside a range (a group commit's intermediate versions are never
@@ -359,7 +360,6 @@ static __device__ void complete_range(uint32_t* done, uint32_t done_mask, Global
   __syncwarp();
   uint32_t busy = 0;
   if (lane == 0) {
-    fence_acq_rel_gpu();
     const uint32_t wl = lo >> 5, wh = hi >> 5, up = FULL >> (31u - (hi & 31u)), dn = FULL << (lo & 31u);
     if (wh != wl) {
       atomicOr(&done[wh & done_mask], up);
@@ -1089,7 +1089,8 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   if (own1) pub1 = install(s1, a[1], vic1);
   // one fence releases both words (a fence then relaxed stores is a release): two release
   // stores in a row would wait for the first to land before the second
-  if (own0 || own1) fence_acq_rel_gpu();
+  __syncwarp();
+  fence_acq_rel_gpu();  // (lane 0's orders every lane's install before the completion bits too)
   if (own0) st_relaxed_gpu(&p.cw[a[0]], (unsigned long long)(pub0 ? pub0 : st0));
   if (own1) st_relaxed_gpu(&p.cw[a[1]], (unsigned long long)(pub1 ? pub1 : st1));
 
@@ -1128,7 +1129,9 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
 // with its stamp, lock the written accounts (lowest lane first, in address order, no waiting), drop
 // the lanes that read what a lower locked lane writes, draw timestamps from the commit server,
 // check that the stamps have not moved, install, publish the stamps. Returns the committed lanes.
-// *tried: locks were tried; *lost: one was held by another warp.
+// *tried: locks were tried; *lost: one was held by another warp. firm: locks on accounts that are
+// only read are waited for at the validation, not shied away from (every 16th attempt of a round:
+// waits point to smaller timestamps, so then someone commits whatever the others' timing is).
 // Bound by its chain of L2 round trips and fences (about 0.65 us a trip): loads that do not
 // depend on each other go out together, the victims' slots are read while the server draws, and
 // one pass over the candidates replaces the two all-pairs loops of TXWriteOverlap and
@@ -1136,16 +1139,17 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
 template <int DEPTH, int MAXR, int MAXW, bool CLUSTER>
 __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm,
                                   MailSlot<MAXR, MAXW>& ms, uint32_t me, uint32_t t, uint32_t op,
-                                  uint32_t nr, const uint32_t (&a)[MAXR], bool mine, uint32_t snap,
+                                  uint32_t nr, const uint32_t (&a)[MAXR], bool mine, bool firm,
                                   uint32_t& seq, bool& tried, bool& lost, bool& failed) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = lane_id();
   const VersionStore vs{p.slots, p.n_items};
   // 1. latest versions and their stamps; a batch of reads in flight together
   constexpr int kBatch = DEPTH <= 4 ? 4 : 2;
+  const uint32_t shy = firm ? 0u : FULL;
   int32_t v[MAXR];
   uint32_t stv[MAXR];
-  bool aborted = false;
+  bool aborted = false, held = false;  // held: an account is locked by another warp
 #pragma unroll
   for (int k0 = 0; k0 < MAXR; k0 += kBatch) {
     SlotEditor<DEPTH> e[kBatch]{};
@@ -1161,6 +1165,8 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
       const int k = k0 + j;
       v[k] = 0;
       stv[k] = (uint32_t)w[j];
+      const uint32_t o = (uint32_t)(w[j] >> 32);
+      held |= (k < 2 ? o : o & shy) != 0u && o != me;
       // the stamp's version not visible yet (word and slots came together): the word again,
       // then the slots after it
       if (mine && k < (int)nr && !e[j].find(stv[k], v[k]))
@@ -1190,16 +1196,25 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   }
   const uint32_t nwm = __ballot_sync(FULL, nowrite);
   const uint32_t agm = __ballot_sync(FULL, mine && aborted);
-  uint32_t cand = __ballot_sync(FULL, has_w);
+  //    A lane that saw a lock on an account it uses sits out: one it writes cannot be locked, one
+  //    it reads most likely moves before the validation, and meanwhile the lane would keep its
+  //    own locks from lanes that can commit. (Seen again beside the first CAS, below. With 2280
+  //    warps on a hot region - 3000 accounts drawing 30 % - the two checks took 2.1 M lost locks
+  //    and 280 K failed validations of a run to 0.9 M and 26 K, 3.5 ms to 1.25.)
+  const uint32_t writers = __ballot_sync(FULL, has_w);
+  uint32_t cand = __ballot_sync(FULL, has_w && !held);
   if (lane == 0) {
     stat_add(sm.stat, ST_COMMIT_NOWRITE, __popc(nwm));
     stat_add(sm.stat, ST_ABORT_DATA_AGE, __popc(agm));
     stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(stm));
+    if (cand == 0u) stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(writers));
   }
+  tried = writers != 0u;
+  lost = writers != cand;
   if (cand == 0u) return nwm;
   // 3. lower candidates that write what this lane writes (overlap) or reads (conflict)
   uint32_t overlap = 0, conflict = 0;
-  const uint32_t nr_max = __reduce_max_sync(FULL, has_w ? nr : 0u);
+  const uint32_t nr_max = __reduce_max_sync(FULL, nr);
   for (uint32_t m = cand; m & (m - 1u); m &= m - 1u) {  // (the highest has none above it)
     const uint32_t i = __ffs(m) - 1u;
     const uint32_t x0 = __shfl_sync(FULL, a[0], i), x1 = __shfl_sync(FULL, a[1], i);
@@ -1217,20 +1232,40 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   //    lower lane that could not lock. In address order, no waiting: the higher one is tried
   //    only once the lower one is held, so two warps never each hold one of the other's pair
   //    (that lock-step was a livelock); a lost lock releases what was taken and backs off.
-  const bool attempt = has_w && overlap == 0u;
-  const bool two = a[0] != a[1];
-  const uint32_t lo_a = min(a[0], a[1]), hi_a = max(a[0], a[1]);
+  //    The CAS is of the whole word, from the stamp read and no owner: an account written since
+  //    is found here and not at the validation, after a timestamp was drawn. Every access of
+  //    this mode to a commit word is a full 8-byte access.
+  const bool attempt = has_w && !held && overlap == 0u;
+  const bool two = a[0] != a[1], up = a[0] < a[1];
+  const unsigned long long free0 = stv[0], free1 = stv[1], own = (unsigned long long)me << 32;
+  unsigned long long* const lo_w = &p.cw[up ? a[0] : a[1]];
+  unsigned long long* const hi_w = &p.cw[up ? a[1] : a[0]];
+  const unsigned long long lo_f = up || !two ? free0 : free1, hi_f = up ? free1 : free0;
   bool got = false;
   if (attempt) {
-    got = atomicCAS(owner_word(p.cw, lo_a), 0u, me) == 0u;
-    if (got && two && atomicCAS(owner_word(p.cw, hi_a), 0u, me) != 0u) {
-      st_relaxed_gpu(owner_word(p.cw, lo_a), 0u);
+    unsigned long long word[MAXR];  // the other accounts', in flight with the CAS
+#pragma unroll
+    for (int k = 2; k < MAXR; k++) word[k] = k < (int)nr ? ld_relaxed_gpu(&p.cw[a[k]]) : 0ull;
+    got = atomicCAS(lo_w, lo_f, lo_f | own) == lo_f;
+    bool stale = false;
+#pragma unroll
+    for (int k = 2; k < MAXR; k++) {
+      // (a load may come after another lane's CAS: a lock of this warp is left to the lane order
+      // below, else two lanes that read what the other writes give way to each other for ever)
+      const uint32_t o = (uint32_t)(word[k] >> 32);
+      stale |= k < (int)nr && ((uint32_t)word[k] != stv[k] || ((o & shy) != 0u && o != me));
+    }
+    if (got && stale) {
+      st_relaxed_gpu(lo_w, lo_f);
+      got = false;
+    }
+    if (got && two && atomicCAS(hi_w, hi_f, hi_f | own) != hi_f) {
+      st_relaxed_gpu(lo_w, lo_f);
       got = false;
     }
   }
   const uint32_t locked = __ballot_sync(FULL, got);
-  tried = true;
-  lost = __any_sync(FULL, attempt && !got);
+  lost |= __any_sync(FULL, attempt && !got);
   // a lane commits unless a lower committing lane of its own warp wrote what it read (their
   // locks have the same owner): the lanes without a conflict do, the others in lane order
   conflict &= locked;
@@ -1238,11 +1273,11 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   for (uint32_t m = locked & ~pass; m; m &= m - 1u)
     pass |= __ballot_sync(FULL, lane == (uint32_t)__ffs(m) - 1u && (conflict & pass) == 0u);
   if (got && !((pass >> lane) & 1u)) {
-    st_relaxed_gpu(owner_word(p.cw, lo_a), 0u);
-    if (two) st_relaxed_gpu(owner_word(p.cw, hi_a), 0u);
+    st_relaxed_gpu(lo_w, lo_f);
+    if (two) st_relaxed_gpu(hi_w, hi_f);
   }
   if (lane == 0) {
-    stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(cand & ~locked));
+    stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(writers & ~locked));
     stat_add(sm.stat, p.prevalidate ? ST_ABORT_PREVALID : ST_ABORT_READ_WRITE, __popc(locked & ~pass));
   }
   cand = pass;
@@ -1253,7 +1288,7 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   seq++;
   __syncwarp();
   if (lane == 0) {
-    ms.snap = snap;
+    ms.snap = 0u;
     ms.cand = cand;
     mail_release<CLUSTER>(&ms.req, seq);
   }
@@ -1281,19 +1316,20 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   //    (Every lane acquired the reply, which orders the validation after the draw.)
   const uint32_t base = ms.base, my_ts = base + 1u + __popc(cand & lanemask_lt());
   if (cand_me) {
-    st_relaxed_gpu(owner_word(p.cw, a[0]), kPendingFlag | my_ts);
-    if (two) st_relaxed_gpu(owner_word(p.cw, a[1]), kPendingFlag | my_ts);
+    st_relaxed_gpu(&p.cw[a[0]], lock_word(stv[0], kPendingFlag | my_ts));
+    if (two) st_relaxed_gpu(&p.cw[a[1]], lock_word(stv[1], kPendingFlag | my_ts));
   }
   // 7. validation: the stamps must not have moved, and a lock held by a transaction earlier in
   //    the order (or one whose timestamp is not known yet) must be resolved first. Waits only
   //    ever point to smaller timestamps: no cycles.
-  bool valid = cand_me;
+  //    The two locked accounts need none: their locks were taken at the stamps read.
+  bool valid = cand_me && (two || stv[0] == stv[1]);
   if (cand_me) {
     unsigned long long word[MAXR];
 #pragma unroll
-    for (int k = 0; k < MAXR; k++) word[k] = k < (int)nr ? ld_relaxed_gpu(&p.cw[a[k]]) : 0ull;
+    for (int k = 2; k < MAXR; k++) word[k] = k < (int)nr ? ld_relaxed_gpu(&p.cw[a[k]]) : 0ull;
 #pragma unroll
-    for (int k = 0; k < MAXR; k++) {
+    for (int k = 2; k < MAXR; k++) {
       if (k >= (int)nr || !valid) continue;
       unsigned long long wd = word[k];
       bool settled = false;
@@ -1320,14 +1356,15 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
     st_relaxed_gpu(p.slots + (size_t)a[0] * DEPTH + vic0, pack_version(my_ts, two ? w0 : w1));
     if (two) st_relaxed_gpu(p.slots + (size_t)a[1] * DEPTH + vic1, pack_version(my_ts, w1));
   }
-  fence_acq_rel_gpu();
+  __syncwarp();
+  fence_acq_rel_gpu();  // (lane 0's orders every lane's install before the completion bits too)
   if (cand_me) {
     if (valid) {
       st_relaxed_gpu(&p.cw[a[0]], (unsigned long long)my_ts);
       if (two) st_relaxed_gpu(&p.cw[a[1]], (unsigned long long)my_ts);
     } else {
-      st_relaxed_gpu(owner_word(p.cw, a[0]), 0u);
-      if (two) st_relaxed_gpu(owner_word(p.cw, a[1]), 0u);
+      st_relaxed_gpu(&p.cw[a[0]], free0);
+      if (two) st_relaxed_gpu(&p.cw[a[1]], free1);
     }
   }
   if (p.log && cand_me) {
@@ -1425,7 +1462,11 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
       if (lane == 0) atomicAdd(&sm.stat[ST_ROUNDS], 1ull);
       tries += (pending >> lane) & 1u;
       if (lock_fails) {  // randomized, growing back-off after a lost lock: breaks lock-step retries
-        const uint32_t h = (me * 0x9E3779B1u) ^ (attempts * 0x85EBCA6Bu);
+        // (mixed after the two are joined: joined by XOR alone, two warps' pauses differ by one
+        // constant in every attempt, and a small one kept them in lock-step until the guard)
+        uint32_t h = me * 0x9E3779B1u + attempts;
+        h = (h ^ (h >> 16)) * 0x85EBCA6Bu;
+        h = (h ^ (h >> 13)) * 0xC2B2AE35u;
         __nanosleep((h >> 16) & ((64u << lock_fails) - 1u));
       }
       if (p.backoff && attempts > 0) {  // a scheduler's per-transaction pause before a retry
@@ -1441,17 +1482,20 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
       ReadSet<MAXR> rs;
       WriteSet<MAXW> ws;
       uint32_t snap = 0, err = 0;
-      if (lane == 0) {  // the device error word beside the clock: no round trip of its own
-        err = ld_relaxed_gpu(&p.gs->error);
-        snap = TXBegin(&p.gs->clock, rs, ws);
+      // the device error word: looked at after an attempt that needs no snapshot, so that its
+      // load is in flight with the attempt's own, else beside the clock
+      if (lane == 0) err = ld_relaxed_gpu(&p.gs->error);
+      const bool latest = stamp && !ro && p.prevalidate != 2;  // reads the newest versions
+      if (!latest) {
+        if (lane == 0) snap = TXBegin(&p.gs->clock, rs, ws);
+        snap = __shfl_sync(0xFFFFFFFFu, snap, 0);
+        if (__shfl_sync(0xFFFFFFFFu, err, 0) != 0u) {  // broadcast: the warp leaves the loop together
+          failed = true;
+          break;
+        }
       }
       rs.n = 0;
       ws.n = 0;
-      snap = __shfl_sync(0xFFFFFFFFu, snap, 0);
-      if (__shfl_sync(0xFFFFFFFFu, err, 0) != 0u) {  // broadcast: the warp leaves the loop together
-        failed = true;
-        break;
-      }
       bool aborted = false;
 
       if (ro) {  // read-only: consistent snapshot read, commits without validation
@@ -1486,6 +1530,7 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
             p, sm, ms, *gx, me, t, op, nr, a, mine, seq, sat_outs >= 2u, gave_up, failed,
             waited, sat);
         sat_outs = sat ? sat_outs + 1u : 0u;
+        failed |= __shfl_sync(0xFFFFFFFFu, err, 0) != 0u;
         if (failed) break;
         if (p.txn_waits && waited) p.txn_waits[t] = 1u;
         if (lane == 0 && gave_up) stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(pending));
@@ -1504,7 +1549,8 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
       if (stamp && p.prevalidate != 2) {  // one transaction per commit
         bool lost = false, tried = false;
         const uint32_t fin = stamp_attempt<DEPTH, MAXR, MAXW, CLUSTER>(
-            p, sm, ms, me, t, op, nr, a, mine, snap, seq, tried, lost, failed);
+            p, sm, ms, me, t, op, nr, a, mine, (attempts & 15u) == 0u, seq, tried, lost, failed);
+        failed |= __shfl_sync(0xFFFFFFFFu, err, 0) != 0u;
         if (failed) break;
         // back off only when a lock was lost to another warp (not for own-warp overlaps)
         if (tried) lock_fails = lost ? min(lock_fails + 1, 6u) : 0u;
@@ -1751,6 +1797,8 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
               if (li < p.log_cap) atomicOr(&p.grp[li >> 5], 1u << (li & 31u));
             }
           }
+          __syncwarp();
+          fence_acq_rel_gpu();
           complete_range(p.done, p.done_mask, p.gs, base + 1, base + __popc(cand));
         } else {
           // no links: leaders release whatever they locked

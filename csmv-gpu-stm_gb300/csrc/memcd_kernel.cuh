@@ -467,6 +467,8 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
         p.val_out[2 * r] = make_uint4(0, 0, 0, 0);
         p.val_out[2 * r + 1] = make_uint4(0, 0, 0, 0);
       }
+      __syncwarp();
+      fence_acq_rel_gpu();
       complete_range(p.done, p.done_mask, p.gs, base + 1, base + __popc(cand));
       pending &= ~okm;
     }
