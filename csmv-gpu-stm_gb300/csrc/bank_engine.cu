@@ -299,14 +299,30 @@ extern "C" csmv_status csmv_bank_create(const csmv_bank_config* cfg, csmv_bank_t
   return CSMV_OK;
 }
 
+// The version store as csmv_bank_load leaves it: each account's value at timestamp 0 in its first
+// slot, the others empty; a thread writes two slots. Made on the device, 4 B an account (or none)
+// cross the host link instead of 8 B a slot.
+static __global__ void bank_load_kernel(ulonglong2* slots, size_t pairs, uint32_t per_account,
+                                        const int32_t* values, int32_t init) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pairs) return;
+  constexpr unsigned long long kEmpty = 0xFFFFFFFFull << 32;
+  const bool first = i % per_account == 0;
+  const int32_t v = first && values ? values[i / per_account] : init;
+  slots[i] = make_ulonglong2(first ? (unsigned long long)(uint32_t)v : kEmpty, kEmpty);
+}
+
 extern "C" csmv_status csmv_bank_load(csmv_bank_t* h, const int32_t* host_values) {
   if (!h) return CSMV_ERR_INVALID_ARG;
   CSMV_CUDA(cudaSetDevice(h->cfg.device));
   const size_t n = h->cfg.n_accounts, D = h->cfg.version_depth;
-  std::vector<unsigned long long> slots(n * D, 0xFFFFFFFFull << 32);
-  for (size_t i = 0; i < n; i++)
-    slots[i * D] = (uint32_t)(host_values ? host_values[i] : h->cfg.init_value);  // ts 0
-  CSMV_CUDA(cudaMemcpyAsync(h->slots, slots.data(), n * D * 8, cudaMemcpyHostToDevice, h->stream));
+  if (host_values)
+    CSMV_CUDA(cudaMemcpyAsync(h->d_values, host_values, n * 4, cudaMemcpyHostToDevice, h->stream));
+  const size_t pairs = n * D / 2;
+  bank_load_kernel<<<(uint32_t)((pairs + 255) / 256), 256, 0, h->stream>>>(
+      reinterpret_cast<ulonglong2*>(h->slots), pairs, (uint32_t)D / 2u,
+      host_values ? h->d_values : nullptr, h->cfg.init_value);
+  CSMV_CUDA(cudaGetLastError());
   CSMV_CUDA(cudaMemsetAsync(h->cw, 0, n * 8, h->stream));
   CSMV_CUDA(cudaMemsetAsync(h->ring, 0, (size_t)h->cfg.ring_size * 16, h->stream));
   CSMV_CUDA(cudaMemsetAsync(h->done, 0, (size_t)kDoneWords * 4, h->stream));
