@@ -87,19 +87,6 @@ __host__ __device__ __forceinline__ uint32_t memcd_tag_hash(uint32_t h) {
 __device__ __forceinline__ bool key_eq(uint4 a, uint4 b) {
   return a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
 }
-__device__ __forceinline__ uint4 ld_relaxed_gpu_v4(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p)
-               : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed_gpu_v4(uint4* p, uint4 v) {
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x),
-               "r"(v.y), "r"(v.z), "r"(v.w)
-               : "memory");
-}
 __device__ __forceinline__ uint32_t tag_ts(unsigned long long t) { return (uint32_t)(t >> 32); }
 
 // One round of 32 requests (request r on this lane), run until every request has committed.
@@ -269,7 +256,6 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
       // where the tag's hash matches or, without a match, for the LRU timestamps.
       uint32_t stw[kWays];
       unsigned long long pick[kWays];  // tag of each way's latest version
-      unsigned long long other = 0;    // tag of the target's other version
       uint32_t second = 0, used = 0;   // slot of the latest version; ways whose record was read
       bool aborted = false;
       int slot = 0;
@@ -322,12 +308,9 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
             }
           used = 0xFFu;
         }
-#pragma unroll
-        for (int wy = 0; wy < kWays; wy++)
-          if (wy == slot) other = tg[wy * D + ((second >> wy) & 1u ? 0 : 1)];
         fence_acq_rel_gpu();
       }
-      // the lock, by a CAS that also proves the entry's stamp (so its versions are the ones
+      // the lock, by a CAS that also proves the entry's stamp (so its latest version is the one
       // read), beside a second look at the tags: no record that was read has been replaced
       uint32_t target = e0 + (uint32_t)slot, st0 = 0;
       bool got = false;
@@ -366,7 +349,9 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
       }
       if (cand == 0) continue;
       // commit timestamps from the CTA's server; meanwhile the version to replace is withdrawn
-      // (the older one: no reader uses it)
+      // (the older one: no reader uses it). Its tag, which a SET that fails puts back, is read
+      // under the lock: a holder before this one may have withdrawn it and put it back at the same
+      // stamp. The load and its fence pass under the draw.
       seq++;
       __syncwarp();
       if (lane == 0) {
@@ -377,7 +362,6 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
       const uint32_t group = peers & cand, n_group = __popc(group), rank = __popc(group & lanemask_lt());
       target = __shfl_sync(FULL, target, lead);
       st0 = __shfl_sync(FULL, st0, lead);
-      const unsigned long long old_tag = __shfl_sync(FULL, other, lead);
       const uint32_t latest = __shfl_sync(FULL, (second >> slot) & 1u, lead);
       // rank 0 replaces the other version, rank 1 the latest, rank 2 rank 0's, ...
       const uint32_t my_slot = (rank & 1u) ? latest : 1u - latest;
@@ -385,7 +369,13 @@ __device__ bool memcd_round(const MemcdParams& p, MemcdShared& sm, MemcdMail& ms
       const bool early = inst && my_slot != latest;
       unsigned long long* my_tag = p.tag + (size_t)target * D + my_slot;
       constexpr unsigned long long kNoTag = (unsigned long long)kEmptyTs << 32;
-      if (early) st_relaxed_gpu(my_tag, kNoTag);  // readers: moving
+      unsigned long long old_tag = kNoTag;
+      fence_acq_rel_gpu();  // the leader's, behind its lock: the last holder's tags
+      __syncwarp();
+      if (early) {
+        old_tag = ld_relaxed_gpu(my_tag);
+        st_relaxed_gpu(my_tag, kNoTag);  // readers: moving
+      }
       fence_acq_rel_gpu();
       bool ok_wait = true;
       if (lane == 0)

@@ -157,3 +157,37 @@ def _poll_logged(srv, bid, timeout=30.0):
             return r
         assert time.time() - t0 < timeout, "batch did not complete"
         time.sleep(0.0002)
+
+
+def test_overlapping_batches_of_differing_ticks_keep_both_versions():
+    """SETs of a few dozen keys in two cache sets, in overlapped batches whose LRU ticks come in no
+    order (a SET that fails its validation then often retries in another way): the table, both
+    versions of every entry, equals the commit log replayed one SET at a time."""
+    n_sets, n_b, per = 2, 32, 256
+    rng = np.random.default_rng(5)
+    ticks = rng.permutation(n_b) + 1
+    reqs = [_ids_requests(rng.integers(0, 40, per // 32).repeat(32), 1, seed=i) for i in range(n_b)]
+    with cg.Server(n_sets=n_sets, client_warps=4, arena_requests=1 << 14, max_inflight_sets=1 << 14,
+                   log_cap=1 << 18, serial_batches=0) as srv:
+        srv.start()
+        ids = [srv.submit(r, tick=int(t)) for r, t in zip(reqs, ticks)]
+        assert all(b is not None for b in ids)
+        for b in ids:
+            _poll_logged(srv, b)
+        st = srv.stop()
+        log_txn, base = srv.log()
+        tags, recs = srv.table()
+    assert st.error == 0 and st.commits_update == n_b * per
+    kind, key, val = (np.concatenate([getattr(r, f) for r in reqs]) for f in ("kind", "key", "val"))
+    table = orc.memcd_empty_table(n_sets)
+    done = np.zeros(n_b * per, bool)
+    for i, r in enumerate(log_txn):
+        if r == 0xFFFFFFFF:
+            continue
+        assert not done[r]
+        done[r] = True
+        table = orc.memcd_serial(kind[r:r + 1], key[r:r + 1], val[r:r + 1], int(ticks[r // per]), n_sets, table,
+                                 base + i)[4:]
+    assert done.all()
+    np.testing.assert_array_equal(tags, table[0])
+    np.testing.assert_array_equal(recs.reshape(table[1].shape), table[1])

@@ -1,0 +1,101 @@
+// driver.cpp - CPU runs of the commit kernels' warp code (see csmv_prims.cuh beside it).
+#include <cstring>
+#include <map>
+#include <set>
+
+#include "csmv-gpu-stm_gb300/csrc/memcd_kernel.cuh"
+
+using namespace csmv;
+
+// `warps` client warps of one CTA and its commit server run rounds of 32 requests of a cache of
+// n_sets sets, round r under the LRU tick ticks[r] (as rounds of overlapping batches do). Returns 0,
+// the device error word, or 255 when the run did not end.
+extern "C" int emu_memcd(uint32_t warps, uint32_t rounds, const uint32_t* kind, const uint32_t* key,
+                         const uint32_t* val, const uint32_t* ticks, uint32_t n_sets, uint64_t seed,
+                         uint32_t switch_log2, unsigned long long* tags, uint32_t* recs,
+                         uint32_t* found, uint32_t* val_out, uint32_t* log_txn, uint32_t log_cap,
+                         uint32_t* outcome, uint32_t* final_ts) {
+  std::vector<uint4> k4(rounds * 32), v4(rounds * 64), rec((size_t)n_sets * kWays * kMemcdDepth * 4),
+      vo(rounds * 64);
+  memcpy(k4.data(), key, k4.size() * 16);
+  memcpy(v4.data(), val, v4.size() * 16);
+  memcpy(rec.data(), recs, rec.size() * 16);
+  std::vector<unsigned long long> cw((size_t)n_sets * kWays), stats(ST_COUNT);
+  std::vector<uint32_t> done(1024);
+  static GlobalSync gs;
+  memset((void*)&gs, 0, sizeof(gs));
+  static MemcdShared sm;
+  memset((void*)&sm, 0, sizeof(sm));
+  MemcdParams p{};
+  p.kind = kind;
+  p.key = k4.data();
+  p.val = v4.data();
+  p.n_rounds = rounds;
+  p.n_sets = n_sets;
+  p.tag = tags;
+  p.rec = rec.data();
+  p.cw = cw.data();
+  p.done = done.data();
+  p.done_mask = 1023;
+  p.gs = &gs;
+  p.found = found;
+  p.val_out = vo.data();
+  p.log_txn = log_txn;
+  p.outcome = outcome;
+  p.log = 1;
+  p.log_cap = log_cap;
+  p.stats = stats.data();
+  p.nc = warps;
+  p.spin_log2 = 30;
+  emu::reset();
+  emu::switch_log2 = switch_log2;
+  emu::add_warp(0, 0, [&] {  // the commit server, one lane: the next timestamps to each request
+    std::vector<uint32_t> seen(warps);
+    for (; lane_id() == 0 && sm.done_warps != warps; emu::pause())
+      for (uint32_t w = 0; w < warps; w++) {
+        const uint32_t req = ld_acquire_cta(&sm.mail[w].req);
+        if (req == seen[w]) continue;
+        sm.mail[w].base = atomicAdd(&gs.ts_next, (uint32_t)__popc(sm.mail[w].cand));
+        st_release_cta(&sm.mail[w].rep, seen[w] = req);
+      }
+  });
+  for (uint32_t w = 0; w < warps; w++)
+    emu::add_warp(0, w + 1, [&, w] {
+      uint32_t seq = 0;
+      for (;;) {
+        uint32_t g = 0;
+        if (lane_id() == 0) g = atomicAdd(&gs.round_next, 1u);
+        g = __shfl_sync(0xFFFFFFFFu, g, 0);
+        if (g >= rounds) break;
+        if (!memcd_round(p, sm, sm.mail[w], w + 1, g * 32u + lane_id(), seq, ticks[g])) break;
+      }
+      __syncwarp();
+      if (lane_id() == 0) atomicAdd(&sm.done_warps, 1u);
+    });
+  // What makes failing SETs meet: a warp that reads a withdrawn tag waits there until its holder
+  // has let go of the entry; one that has locked an entry waits until a stamp of the set moves.
+  auto in = [](const void* q, const auto& v) { return q >= v.data() && q < v.data() + v.size(); };
+  emu::on_load = [&](const void* q, bool) {
+    const unsigned long long* t = (const unsigned long long*)q;
+    if (t < tags || t >= tags + cw.size() * kMemcdDepth || tag_ts(*t) != kEmptyTs) return;
+    const unsigned long long* w = &cw[(t - tags) / kMemcdDepth];
+    if ((*w >> 32) != 0ull && (emu::rnd() & 3u)) emu::hold([w] { return (*w >> 32) == 0ull; }, 60000);
+  };
+  emu::on_store = [&](const void* q, unsigned long long v) {
+    const uint32_t own = (uint32_t)(v >> 32);
+    if (!in(q, cw) || own == 0u || (own & kPendingFlag) || (emu::rnd() & 1u) == 0u) return;
+    const size_t e0 = ((const unsigned long long*)q - cw.data()) / kWays * kWays;
+    const std::vector<unsigned long long> was(cw.begin() + e0, cw.begin() + e0 + kWays);
+    emu::cur->warp->until = [&cw, e0, was] {
+      for (int i = 0; i < kWays; i++)
+        if ((uint32_t)cw[e0 + i] != (uint32_t)was[i]) return true;
+      return false;
+    };
+    emu::cur->warp->patience = emu::steps + 8000;
+  };
+  const bool ended = emu::run(seed, 1ull << 28);
+  memcpy(recs, rec.data(), rec.size() * 16);
+  memcpy(val_out, vo.data(), vo.size() * 16);
+  *final_ts = gs.ts_next;
+  return ended ? (int)gs.error : 255;
+}
