@@ -315,7 +315,9 @@ struct SlotEditor {
 // snapshot may take), at most over the whole bitmap, which holds every timestamp in flight.
 // Words read together are not ordered, so a scan that stops at a word's first bit - where a
 // range's upper part may be missing - reads that word again. w: the lanes' words from word
-// first on, read already. Warp-collective; the caller fences before it publishes the end.
+// first on, read already. Warp-collective. Every lane fences behind the words that it read, which
+// makes them acquires: the write-backs behind them come before the clock that the caller
+// publishes (with a fence of its own, after a warp barrier).
 static __device__ uint32_t complete_prefix(const uint32_t* done, uint32_t done_mask, uint32_t c,
                                            uint32_t first, uint32_t w) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -328,16 +330,19 @@ static __device__ uint32_t complete_prefix(const uint32_t* done, uint32_t done_m
     have = false;
     if (lane == 0) w |= (1u << ((n + 1u) & 31u)) - 1u;
     const uint32_t open = __ballot_sync(FULL, w != FULL);
+    bool last = false;
     if (open == 0u) {
       n = ((first + 32u) << 5) - 1u;
     } else {
       const uint32_t k = __ffs(open) - 1u;
       const uint32_t b = __ffs(~__shfl_sync(FULL, w, k)) - 1u;
       n = ((first + k) << 5) + b - 1u;
-      if (b != 0u || k == 0u) break;
+      last = b != 0u || k == 0u;
     }
-    fence_acq_rel_gpu();  // the words of the next step are read after these
+    if (n == c) break;  // (nothing to publish)
+    fence_acq_rel_gpu();  // (the words of the next step are read after these, too)
     __syncwarp();
+    if (last) break;
   }
   return n;
 }

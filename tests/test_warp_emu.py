@@ -37,6 +37,7 @@ def emu(tmp_path_factory):
     so = C.CDLL(str(lib))
     P, U = C.c_void_p, C.c_uint32
     so.emu_memcd.argtypes = [U, U, P, P, P, P, U, C.c_uint64, U, P, P, P, P, P, U, P, P]
+    so.emu_complete.argtypes = [U, U, P, P, U, U, C.c_uint64, P, P]
     return so
 
 
@@ -84,3 +85,21 @@ def test_cache_versions_survive_failed_sets(emu, seed):
         np.testing.assert_array_equal(tags, table[0])
         np.testing.assert_array_equal(recs, table[1])
     assert holes > 0  # validations did fail
+
+
+@pytest.mark.parametrize("warps", [1, 2, 5])
+@pytest.mark.parametrize("clock0", [0, 31, 4000])
+def test_clock_covers_only_acquired_completions(emu, warps, clock0):
+    """The warp that moves the clock has acquired, in each lane, the completion words it moves it
+    over: what a snapshot at the new clock reads was written back before. The clock ends behind the
+    last range."""
+    rng = np.random.default_rng(clock0 + warps)
+    for seed in range(5):
+        end = clock0 + np.cumsum(rng.integers(1, 33, 100))
+        lo = np.concatenate([[clock0], end[:-1]]) + 1
+        perm = rng.permutation(100)
+        lo, hi = lo[perm].astype(np.uint32), end[perm].astype(np.uint32)
+        fin, bad = C.c_uint32(), C.c_uint32()
+        assert emu.emu_complete(warps, 100, p(lo), p(hi), clock0, 127, seed, C.byref(fin), C.byref(bad)) == 0
+        assert fin.value == end[-1]
+        assert bad.value == 0

@@ -99,3 +99,42 @@ extern "C" int emu_memcd(uint32_t warps, uint32_t rounds, const uint32_t* kind, 
   *final_ts = gs.ts_next;
   return ended ? (int)gs.error : 255;
 }
+
+// `warps` warps complete the ranges [lo[i], hi[i]] of timestamps after clock0, warp w those with
+// i = w, w + warps, ... Counts in *unordered the completion words that a clock store passes while the
+// lane that read them has not acquired them (a fence, or the load itself). Returns 0, or 255 when
+// the run did not end.
+extern "C" int emu_complete(uint32_t warps, uint32_t n, const uint32_t* lo, const uint32_t* hi,
+                            uint32_t clock0, uint32_t done_mask, uint64_t seed, uint32_t* clock_end,
+                            uint32_t* unordered) {
+  std::vector<uint32_t> done(done_mask + 1);
+  static GlobalSync gs;
+  memset((void*)&gs, 0, sizeof(gs));
+  gs.clock = clock0;
+  *unordered = 0;
+  emu::reset();
+  emu::switch_log2 = 2;
+  for (uint32_t w = 0; w < warps; w++)
+    emu::add_warp(0, w, [&, w] {
+      for (uint32_t i = w; i < n; i += warps) complete_range(done.data(), done_mask, &gs, lo[i], hi[i]);
+    });
+  std::map<const emu::Lane*, std::set<uint32_t>> open;  // words read and not acquired yet
+  emu::on_load = [&](const void* q, bool acquire) {
+    const uint32_t* d = (const uint32_t*)q;
+    if (d < done.data() || d > done.data() + done_mask) return;
+    if (acquire)
+      open[emu::cur].erase(d - done.data());
+    else
+      open[emu::cur].insert(d - done.data());
+  };
+  emu::on_fence = [&] { open[emu::cur].clear(); };
+  emu::on_store = [&](const void* q, unsigned long long v) {
+    if (q != &gs.clock) return;
+    for (auto& [lane, words] : open)
+      if (lane->warp == emu::cur->warp)
+        for (uint32_t t = (gs.clock + 1u) >> 5; t <= (uint32_t)v >> 5; t++) *unordered += words.count(t & done_mask);
+  };
+  const bool ended = emu::run(seed, 1ull << 26);
+  *clock_end = gs.clock;
+  return ended ? 0 : 255;
+}
