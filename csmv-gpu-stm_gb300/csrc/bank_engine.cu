@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "bank_internal.h"
+#include "tune_pick.h"
 
 using namespace csmv;
 
@@ -803,9 +804,10 @@ extern "C" csmv_status csmv_bank_autotune(const csmv_bank_config* base,
     std::sort(m.begin(), m.end());
     t.best_ms = m[m.size() / 2];  // median over every run
   }
-  size_t best = order[0];
-  for (size_t r = 0; r < keep; r++)
-    if (trials[order[r]].st == CSMV_OK && trials[order[r]].best_ms < trials[best].best_ms) best = order[r];
+  std::vector<double> ms;
+  for (const Trial& t : trials) ms.push_back(t.st == CSMV_OK ? t.best_ms : 1e30);
+  order.resize(keep);
+  const size_t best = tune_pick(order, ms);
   if (trials[best].st != CSMV_OK) {
     set_error("autotune: no candidate ran (%s)", csmv_status_str(trials[best].st));
     return trials[best].st;

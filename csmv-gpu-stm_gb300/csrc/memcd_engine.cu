@@ -15,6 +15,7 @@
 
 #include "common.h"
 #include "memcd_kernel.cuh"
+#include "tune_pick.h"
 
 using namespace csmv;
 
@@ -385,9 +386,10 @@ extern "C" csmv_status csmv_memcd_autotune(const csmv_memcd_config* base,
     std::sort(m.begin(), m.end());
     c.med = m[m.size() / 2];
   }
-  size_t best = order[0];
-  for (size_t r = 0; r < keep; r++)
-    if (cands[order[r]].st == CSMV_OK && cands[order[r]].med < cands[best].med) best = order[r];
+  std::vector<double> ms;
+  for (const Cand& c : cands) ms.push_back(c.st == CSMV_OK ? c.med : 1e30);
+  order.resize(keep);
+  const size_t best = tune_pick(order, ms);
   if (cands[best].st != CSMV_OK) {
     set_error("memcd autotune: no candidate ran (%s)", csmv_status_str(cands[best].st));
     return cands[best].st;
