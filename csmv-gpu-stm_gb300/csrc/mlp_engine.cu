@@ -193,6 +193,10 @@ csmv_status csmv_mlp_forward_status(csmv_mlp_t* h) {
 extern "C" csmv_status csmv_mlp_forward(csmv_mlp_t* h, uint32_t n, const uint16_t* dev_x,
                                         float* dev_p) {
   if (!h || (n && (!dev_x || !dev_p))) return CSMV_ERR_INVALID_ARG;
+  if (n && (reinterpret_cast<uintptr_t>(dev_x) & 15u)) {  // a misaligned 16-byte copy is a fault
+    set_error("csmv_mlp_forward: the features must begin on a 16-byte boundary");
+    return CSMV_ERR_INVALID_ARG;
+  }
   CSMV_CUDA(cudaSetDevice(h->device));
   csmv_status st = csmv_mlp_launch_forward(h, n, dev_x, dev_p, h->stream);
   if (st != CSMV_OK) return st;

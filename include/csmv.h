@@ -543,10 +543,11 @@ typedef struct csmv_mlp_t csmv_mlp_t;
 csmv_status csmv_mlp_create(int32_t device, uint64_t seed, csmv_mlp_t** out);
 csmv_status csmv_mlp_set_params(csmv_mlp_t* m, const float* host_params); /* resets Adam */
 csmv_status csmv_mlp_get_params(csmv_mlp_t* m, float* host_params);
-/* dev_p[i] = predicted abort probability of sample i */
+/* dev_p[i] = predicted abort probability of sample i. dev_x is on a 16-byte boundary (rows are
+ * copied in 16-byte pieces), else CSMV_ERR_INVALID_ARG. */
 csmv_status csmv_mlp_forward(csmv_mlp_t* m, uint32_t n, const uint16_t* dev_x, float* dev_p);
 /* Adds the gradient of the mean loss over the n samples to the handle's accumulator;
- * *host_loss (optional) = that mean loss. */
+ * *host_loss (optional) = that mean loss. dev_x may begin at any element. */
 csmv_status csmv_mlp_grad(csmv_mlp_t* m, uint32_t n, const uint16_t* dev_x, const float* dev_y,
                           float* host_loss);
 csmv_status csmv_mlp_get_grads(csmv_mlp_t* m, float* host_grads);

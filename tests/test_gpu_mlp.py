@@ -164,3 +164,23 @@ def test_gradient_at_tile_and_grid_edges(n, offset):
     loss_ref, g_ref = mo.loss_and_grads(params, x, y)
     assert max(abs(l - loss_ref) for l in losses) < 1e-4 * max(1.0, abs(loss_ref))
     np.testing.assert_allclose(g, g_ref, rtol=0, atol=1e-4 * np.abs(g_ref).max())
+
+
+@pytest.mark.parametrize("offset", [1, 4, 7, 8, 15])
+def test_forward_refuses_features_off_a_16_byte_boundary(offset):
+    """Inference copies its features in 16-byte pieces: a pointer between two of them is refused on
+    the host (the gradient takes it), one on a boundary inside an allocation is not."""
+    torch = pytest.importorskip("torch")
+    n = 130
+    x, xb = _features(np.random.default_rng(offset), n)
+    with cg.Mlp(seed=5) as m:
+        whole = torch.zeros(offset + n * mo.IN, dtype=torch.int16, device="cuda")
+        whole[offset:] = _dev(torch, xb).flatten()
+        dp = torch.full((n,), 7.0, device="cuda")
+        if offset % 8:
+            with pytest.raises(cg.CsmvError) as e:
+                m.forward(n, whole.data_ptr() + 2 * offset, dp.data_ptr())
+            assert e.value.status == 1 and (dp == 7.0).all()
+        else:
+            m.forward(n, whole.data_ptr() + 2 * offset, dp.data_ptr())
+            np.testing.assert_allclose(dp.cpu().numpy(), mo.forward(m.params(), x)[0], rtol=0, atol=2e-5)
