@@ -1180,12 +1180,14 @@ __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   }
   // 2. the transfer. One that writes nothing is read-only: it serialises at the largest stamp it
   //    read, once a second collect finds every stamp unchanged and no lock on them (a writer of
-  //    one of them with a smaller timestamp would hold its lock)
+  //    one of them with a smaller timestamp would hold its lock). A fence keeps the collects
+  //    apart: what the first one saw of a commit, the second one sees the lock or stamp of.
   int32_t w0 = 0, w1 = 0;
   const bool has_w = mine && !aborted && transfer_writes<MAXR>(op, nr, v, w0, w1);
   bool nowrite = mine && !aborted && !has_w;
   uint32_t ro_snap = 0;
   bool moved = false;
+  if (nowrite) fence_acq_rel_gpu();
 #pragma unroll
   for (int k = 0; k < MAXR; k++) {
     if (!nowrite || k >= (int)nr) continue;

@@ -38,6 +38,7 @@ def emu(tmp_path_factory):
     P, U = C.c_void_p, C.c_uint32
     so.emu_memcd.argtypes = [U, U, P, P, P, P, U, C.c_uint64, U, P, P, P, P, P, U, P, P]
     so.emu_complete.argtypes = [U, U, P, P, U, U, C.c_uint64, P, P]
+    so.emu_short_funds.argtypes, so.emu_short_funds.restype = [U, P, P, U, P, C.c_uint64, P], U
     return so
 
 
@@ -103,3 +104,17 @@ def test_clock_covers_only_acquired_completions(emu, warps, clock0):
         assert emu.emu_complete(warps, 100, p(lo), p(hi), clock0, 127, seed, C.byref(fin), C.byref(bad)) == 0
         assert fin.value == end[-1]
         assert bad.value == 0
+
+
+@pytest.mark.parametrize("nr", [2, 3, 8])
+def test_transfers_without_funds_look_twice_behind_a_fence(emu, nr):
+    """A transfer that writes nothing commits on two looks at its accounts' commit words; a fence
+    of the lane lies between them."""
+    rng = np.random.default_rng(nr)
+    addr = rng.permuted(np.tile(np.arange(40), (32, 1)), axis=1)[:, :nr].astype(np.uint32)
+    op = np.full(32, cg.KIND_TRANSFER | nr << 2 | 5 << 8 | 4095 << 20, np.uint32)
+    value = np.full(40, 4, np.int32)
+    addr = np.ascontiguousarray(addr)
+    bad = C.c_uint32()
+    assert emu.emu_short_funds(nr, p(op), p(addr), 40, p(value), 1, C.byref(bad)) == 0xFFFFFFFF
+    assert bad.value == 0

@@ -138,3 +138,45 @@ extern "C" int emu_complete(uint32_t warps, uint32_t n, const uint32_t* lo, cons
   *clock_end = gs.clock;
   return ended ? 0 : 255;
 }
+
+// One attempt of the per-transaction protocol for a round of transfers of nr accounts each (addr
+// [32][nr]) whose funds are short, beside nothing else. Counts in *unordered the commit words that a
+// lane looks at again without a fence since its first look. Returns the committed lanes.
+extern "C" uint32_t emu_short_funds(uint32_t nr, const uint32_t* op, const uint32_t* addr, uint32_t n_items,
+                                    const int32_t* value, uint64_t seed, uint32_t* unordered) {
+  constexpr int kD = 4, kR = 8;
+  std::vector<unsigned long long> slots((size_t)n_items * kD, 0xFFFFFFFFull << 32), cw(n_items), stats(ST_COUNT);
+  for (uint32_t i = 0; i < n_items; i++) slots[(size_t)i * kD] = (uint32_t)value[i];
+  static GlobalSync gs;
+  memset((void*)&gs, 0, sizeof(gs));
+  static CtaShared<kR, 2> sm;
+  memset((void*)&sm, 0, sizeof(sm));
+  std::vector<uint32_t> outcome(32);
+  std::vector<int32_t> result(32);
+  BankParams p{};
+  p.n_items = n_items;
+  p.slots = slots.data();
+  p.cw = cw.data();
+  p.gs = &gs;
+  p.outcome = outcome.data();
+  p.result = (int32_t*)result.data();
+  p.log = 1;
+  p.prevalidate = 1;
+  p.spin_log2 = 20;
+  uint32_t fin = 0;
+  *unordered = 0;
+  emu::reset();
+  emu::add_warp(0, 1, [&] {
+    uint32_t a[kR] = {}, seq = 0;
+    for (uint32_t k = 0; k < nr; k++) a[k] = addr[lane_id() * nr + k];
+    bool tried = false, lost = false, failed = false;
+    fin = stamp_attempt<kD, kR, 2, false>(p, sm, sm.mail[0], 1u, lane_id(), op[lane_id()], nr, a, true, false, seq,
+                                          tried, lost, failed);
+  });
+  std::map<const emu::Lane*, std::set<const void*>> open;  // words looked at, no fence since
+  emu::on_load = [&](const void* q, bool) {
+    if (q >= cw.data() && q < cw.data() + n_items && !open[emu::cur].insert(q).second) ++*unordered;
+  };
+  emu::on_fence = [&] { open[emu::cur].clear(); };
+  return emu::run(seed, 1ull << 24) ? fin : 0u;
+}
