@@ -255,9 +255,12 @@ csmv_status csmv_bank_run_device(csmv_bank_t* h, const csmv_bank_stream* dev_str
  * order of the handle (stamp protocol only). Meant for transactions a scheduler predicts to
  * conflict; no other run of the handle may be in flight. Every transaction commits; read-only
  * ones see the state after all earlier ones. Short streams are run by one warp, a round's 32
- * transfers resolving their dependencies as a chain in lane order; streams of 96 rounds and more
- * by the dataflow lane's kernels (below, with their device scratch), which leave the same
- * state - where these cannot take the stream, by the one warp too. */
+ * transfers resolving their dependencies as a chain in lane order; streams of 96 rounds to 2^22
+ * transactions by the dataflow lane's kernels (below), which leave the same state. The handle
+ * then keeps their device scratch, of about 28 B per access and 40 B per transaction of its
+ * largest run (at most 2 GB), until it is destroyed. Where these kernels cannot take the stream
+ * (more than 2^26 accesses, no memory for the scratch, a malformed round), the one warp runs it:
+ * the rounds before a malformed one are applied. */
 csmv_status csmv_bank_run_serial_device(csmv_bank_t* h, const csmv_bank_stream* dev_stream,
                                         csmv_stats* out);
 

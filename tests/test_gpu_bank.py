@@ -666,3 +666,35 @@ def test_read_widths_on_one_warp_equal_the_model(up_reads, max_reads, prevalidat
         log_txn, outcome, result = bank.log(n, st.final_ts)
         for got, want in zip((bank.versions(), log_txn, outcome, result), model):
             np.testing.assert_array_equal(got, want)
+
+
+def test_serial_lane_past_the_access_limit_runs_on_one_warp():
+    """A serial-lane run of more accesses than the dataflow kernels take goes to the one-warp kernel:
+    every sum is the oracle's, and the dataflow lane's buffers are left alone."""
+    torch = pytest.importorskip("torch")
+    n_acc, few, n, nr = 1024, 32 * 1024, (1 << 20) + (1 << 15), 63  # 68.1 M accesses of at most 2^26
+    s = cg.generate(c1_workload(n_txn=few, n_accounts=n_acc, up_reads=8, pr_read_pct=0, seed=3))
+    rng = np.random.default_rng(3)
+    addr = np.concatenate([s.addr[s.off[0]:s.off[0] + 8 * 32],
+                           rng.integers(0, n_acc, (n - 32) * nr, dtype=np.uint32)]).astype(np.uint32)
+    op = np.concatenate([s.op[:32], np.full(n - 32, nr << 2 | 1 << 8 | 1 << 20, np.uint32)])
+    off = np.concatenate([np.arange(32) * 8, 32 * 8 + np.arange(n - 32, dtype=np.int64) * nr]).astype(np.uint32)
+    assert (s.off[:32] == s.off[0] + 8 * np.arange(32)).all()
+    init = np.full(n_acc, 1000, np.int32)
+    first, _ = orc.serial(s.op, s.off, s.addr, n_acc, init)
+    want, _ = orc.serial(op[:32], off[:32], addr, n_acc, first)
+    sums = want[addr[32 * 8:].reshape(-1, nr)].sum(1, dtype=np.int32)
+    with cg.Bank(n_accounts=n_acc, max_txn=n, version_depth=4) as bank:
+        bank.load()
+        ds, keep = to_device(torch, s)
+        prev = bank.run_flow_device(ds).final_ts
+        dl, keep2 = to_device(torch, cg.Stream(op, off, addr))
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        st = bank.run_serial_device(dl)
+        assert torch.cuda.mem_get_info()[0] <= free
+        _, outcome, result = bank.log(n, st.final_ts - prev)
+        np.testing.assert_array_equal(bank.values(), want)
+    assert st.commits == n and st.aborts == 0
+    np.testing.assert_array_equal(result[32:], sums)
+    assert (outcome[32:] == (st.final_ts | cg.SNAP_FLAG)).all()
