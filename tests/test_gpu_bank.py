@@ -698,3 +698,145 @@ def test_serial_lane_past_the_access_limit_runs_on_one_warp():
     assert st.commits == n and st.aborts == 0
     np.testing.assert_array_equal(result[32:], sums)
     assert (outcome[32:] == (st.final_ts | cg.SNAP_FLAG)).all()
+
+
+def serial_in_pieces(torch, bank, s, rounds=90, lo=0, prev=0):
+    """The stream's rounds from lo on in serial-lane runs short enough for the one-warp kernel:
+    (statistics of the runs, log, outcomes, results, last timestamp), joined over the runs."""
+    stats, logs, outs, ress = [], [], [], []
+    for at in range(32 * lo, s.n_txn, 32 * rounds):
+        end = min(at + 32 * rounds, s.n_txn)
+        ds, keep = to_device(torch, sub_stream(s, at, end))
+        st = bank.run_serial_device(ds)
+        a, b, c = bank.log(end - at, st.final_ts - prev)
+        stats.append(st)
+        logs.append(np.where(a != 0xFFFFFFFF, a + np.uint32(at), a).astype(np.uint32))
+        outs.append(b)
+        ress.append(c)
+        prev = st.final_ts
+    return stats, np.concatenate(logs), np.concatenate(outs), np.concatenate(ress), prev
+
+
+@pytest.mark.parametrize("case", list(FLOW_CASES))
+def test_flow_lane_equals_the_one_warp_kernel(case):
+    """The dataflow lane leaves exactly what the serial lane's one-warp kernel leaves, the stream fed
+    to that one in pieces of 90 rounds: versions in the same slots, log, outcomes, results, sums of
+    the statistics."""
+    torch = pytest.importorskip("torch")
+    c = FLOW_CASES[case]
+    n_acc, n, depth = c["n_acc"], c["n"], c["depth"]
+    s = cg.generate(c1_workload(n_txn=n, n_accounts=n_acc, dist=c["dist"], zipf_theta=0.99,
+                                up_reads=c["up_reads"], pr_read_pct=c["ro"], seed=22,
+                                kind=c.get("kind", cg.KIND_TRANSFER)))
+    if "self_every" in c:
+        t = np.flatnonzero((s.op & 3) != 0)[:: c["self_every"]]
+        s.addr[s.off[t] + 1] = s.addr[s.off[t]]
+    kw = dict(n_accounts=n_acc, max_txn=n, version_depth=depth, flow_warps=c.get("flow_warps", 0))
+    with cg.Bank(**kw) as bank:
+        bank.load()
+        ds, keep = to_device(torch, s)
+        st = bank.run_flow_device(ds)
+        flow = (*bank.log(n, st.final_ts), bank.versions(), bank.values())
+    with cg.Bank(**kw) as bank:
+        bank.load()
+        stats, log, oc, rs, last = serial_in_pieces(torch, bank, s)
+        one_warp = (log, oc, rs, bank.versions(), bank.values())
+    assert st.commits == n and st.aborts == 0 and st.final_ts == last
+    for f in ("commits_update", "commits_readonly", "commits_nowrite", "rounds", "sections"):
+        assert getattr(st, f) == sum(getattr(x, f) for x in stats), f
+    for a, b in zip(flow, one_warp):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("dist", [cg.DIST_UNIFORM, cg.DIST_ZIPF])
+def test_one_warp_serial_runs_equal_stream_order_execution(dist):
+    """The one-warp kernel over 600 rounds, in pieces: final balances of the serial oracle, commits
+    in stream order, exact replay."""
+    torch = pytest.importorskip("torch")
+    n_acc, n = 2048, 32 * 600
+    s = cg.generate(c1_workload(n_txn=n, n_accounts=n_acc, dist=dist, zipf_theta=0.99, up_reads=4,
+                                pr_read_pct=20, seed=12))
+    with cg.Bank(n_accounts=n_acc, max_txn=n, version_depth=4) as bank:
+        bank.load()
+        _, log, outcome, result, last = serial_in_pieces(torch, bank, s)
+        slots, vals = bank.versions(), bank.values()
+    init = np.full(n_acc, 1000, np.int32)
+    err = orc.check(s.op, s.off, s.addr, n_acc, init, 4, last, log, outcome, result, slots)
+    assert err is None, err
+    np.testing.assert_array_equal(vals, orc.serial(s.op, s.off, s.addr, n_acc, init)[0])
+    writers = np.flatnonzero((outcome & cg.SNAP_FLAG) == 0)
+    assert (log == writers).all()
+
+
+def test_engine_one_warp_and_flow_runs_interleave_exactly():
+    """Concurrent, one-warp serial, dataflow and concurrent runs of 95 rounds each on one bank: the
+    commit order carries across them and the concatenated log replays exactly."""
+    torch = pytest.importorskip("torch")
+    n_acc, n = 4096, 32 * 95  # one round short of the serial lane's change of kernels
+    s = cg.generate(c1_workload(n_txn=6 * n, n_accounts=n_acc, seed=19, dist=cg.DIST_ZIPF, zipf_theta=0.9,
+                                up_reads=4))
+    logs, prev = [], 0
+    with cg.Bank(n_accounts=n_acc, max_txn=n, ctas=8, client_warps=4) as bank:
+        bank.load()
+        runs = (bank.run_device, bank.run_serial_device, bank.run_flow_device, bank.run_serial_device,
+                bank.run_device, bank.run_serial_device)
+        for i, run in enumerate(runs):
+            ds, keep = to_device(torch, sub_stream(s, i * n, (i + 1) * n))
+            st = run(ds)
+            lt, oc, rs = bank.log(n, st.final_ts - prev)
+            logs.append((np.where(lt != 0xFFFFFFFF, lt + np.uint32(i * n), lt).astype(np.uint32), oc, rs))
+            prev = st.final_ts
+        slots = bank.versions()
+    err = orc.check(s.op, s.off, s.addr, n_acc, np.full(n_acc, 1000, np.int32), 4, prev,
+                    *[np.concatenate(x) for x in zip(*logs)], slots)
+    assert err is None, err
+
+
+def test_serial_lane_past_the_transaction_limit_equals_the_flow_lane():
+    """A serial-lane run of more than 2^22 transactions stays with the one-warp kernel; the dataflow
+    lane, which takes up to 2^25, leaves the same state."""
+    torch = pytest.importorskip("torch")
+    n_acc, n = 1 << 14, (1 << 22) + 32
+    s = cg.generate(c1_workload(n_txn=n, n_accounts=n_acc, seed=29, up_reads=2, pr_read_pct=0))
+    ds, keep = to_device(torch, s)
+    got = []
+    with cg.Bank(n_accounts=n_acc, max_txn=n, version_depth=4) as bank:
+        for lane in (bank.run_serial_device, bank.run_flow_device):
+            bank.load()
+            st = lane(ds)
+            assert st.commits == n and st.aborts == 0
+            got.append((st.final_ts, *bank.log(n, st.final_ts), bank.versions()))
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
+    np.testing.assert_array_equal(orc.serial(s.op, s.off, s.addr, n_acc, np.full(n_acc, 1000, np.int32))[0],
+                                  newest(got[0][-1], 4))
+
+
+def newest(slots, depth):
+    """Each account's value of the largest timestamp."""
+    v = slots.reshape(-1, depth)
+    ts = (v >> np.uint64(32)).astype(np.int64)
+    ts[ts == 0xFFFFFFFF] = -1
+    return v[np.arange(len(v)), ts.argmax(1)].astype(np.uint32).view(np.int32)
+
+
+FEW_ROUNDS = [  # validate, write-back, batch, prevalidate
+    (cg.VALIDATE_STAMP, cg.WRITEBACK_CLIENT, cg.BATCH_CTA, 0),
+    (cg.VALIDATE_STAMP, cg.WRITEBACK_CLIENT, cg.BATCH_CTA, 2),
+    (cg.VALIDATE_STAMP, cg.WRITEBACK_CLIENT, cg.BATCH_WARP, 1),
+    (cg.VALIDATE_RING, cg.WRITEBACK_CLIENT, cg.BATCH_CTA, 1),
+    (cg.VALIDATE_RING, cg.WRITEBACK_SERVER, cg.BATCH_CTA, 0),
+    (cg.VALIDATE_RING, cg.WRITEBACK_SERVER, cg.BATCH_LANE, 1),
+    (cg.VALIDATE_RING_LANE, cg.WRITEBACK_SERVER, cg.BATCH_WARP, 1),
+]
+
+
+@pytest.mark.parametrize("rounds", [1, 2, 4, 7, 12])
+@pytest.mark.parametrize("mode", FEW_ROUNDS)
+def test_streams_of_few_rounds_in_every_commit_mode(mode, rounds):
+    """Streams of fewer rounds than the handle has warps, under the commit modes besides the default
+    ones: the smaller launch commits every transaction and replays exactly."""
+    validate, writeback, batch, prevalidate = mode
+    run_checked(c1_workload(n_txn=32 * rounds, n_accounts=512, up_reads=3, pr_read_pct=20, seed=rounds),
+                ctas=3, client_warps=4, validate=validate, writeback=writeback, batch=batch,
+                prevalidate=prevalidate)
