@@ -1581,24 +1581,6 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
             v[k] = TXRead<DEPTH>(vs, a[k], snap, rs, ws, &aborted);
         }
       }
-      // a transfer that commits no writes is read-only: in the stamp protocol it serialises at
-      // the largest stamp it read, once a second collect finds every stamp unchanged and no
-      // lock on them (a writer of one of them with a smaller timestamp would hold its lock)
-      uint32_t ro_snap = snap;
-      auto recheck = [&](bool active) {
-        bool ok = active;
-        uint32_t mx = 0;
-#pragma unroll
-        for (int k = 0; k < MAXR; k++) {
-          if (!active || k >= (int)nr) continue;
-          const unsigned long long wd = ld_relaxed_gpu(&p.cw[a[k]]);
-          ok &= (uint32_t)wd == stv[k] && (uint32_t)(wd >> 32) == 0u;
-          mx = max(mx, stv[k]);
-        }
-        ro_snap = mx;
-        return ok;
-      };
-
       // ---- stamp protocol with intra-warp chaining (prevalidate == 2): instead of aborting a
       // lane that read what a lower lane writes (TXPreValidation), the warp runs its transfers as
       // one serial chain in lane order, forwarding each lower lane's written values to the lanes
@@ -1647,9 +1629,6 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
         // a no-write transfer serialised at the stamps it read could fall inside a chain, whose
         // intermediate states are never installed
         const bool part = okr;
-        const bool ro_cand = false;
-        const bool snap_ok = recheck(ro_cand);
-        const bool ro_fail = ro_cand && !snap_ok;
         // lock leaders: the lowest lane writing each address takes its lock
         uint32_t lead_lane[2] = {lane, lane}, lead_slot[2] = {0u, 1u};
         bool found[2] = {false, false};
@@ -1681,17 +1660,9 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
           F |= __ballot_sync(0xFFFFFFFFu, lane == i && part && (!lock_ok || (fwd & F) != 0));
         const uint32_t partm = __ballot_sync(0xFFFFFFFFu, part);
         const uint32_t lockf = __ballot_sync(0xFFFFFFFFu, part && !lock_ok);
-        const uint32_t snapm = __ballot_sync(0xFFFFFFFFu, snap_ok);
         const uint32_t agm = __ballot_sync(0xFFFFFFFFu, mine && aborted);
-        const uint32_t stm = __ballot_sync(0xFFFFFFFFu, ro_fail);
-        if (snap_ok && p.log) {
-          p.outcome[t] = ro_snap | kSnapFlag;
-          p.result[t] = 0;
-        }
         if (lane == 0) {
-          stat_add(sm.stat, ST_COMMIT_NOWRITE, __popc(snapm));
           stat_add(sm.stat, ST_ABORT_DATA_AGE, __popc(agm));
-          stat_add(sm.stat, ST_ABORT_READ_WRITE, __popc(stm));
           stat_add(sm.stat, ST_ABORT_WRITE_WRITE, __popc(lockf));
           stat_add(sm.stat, ST_ABORT_PREVALID, __popc(F & ~lockf));
         }
@@ -1818,7 +1789,7 @@ __device__ void client_warp(const BankParams& p, CtaShared<MAXR, MAXW>& sm, uint
           stat_add(sm.stat, ST_COMMIT_UPDATE, __popc(hw_c));
           stat_add(sm.stat, ST_COMMIT_NOWRITE, __popc(C & ~hw_c));
         }
-        pending &= ~(C | snapm);
+        pending &= ~C;
         continue;
       }
       bool has_w = false;

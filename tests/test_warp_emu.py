@@ -39,6 +39,7 @@ def emu(tmp_path_factory):
     so.emu_memcd.argtypes = [U, U, P, P, P, P, U, C.c_uint64, U, P, P, P, P, P, U, P, P]
     so.emu_complete.argtypes = [U, U, P, P, U, U, C.c_uint64, P, P]
     so.emu_short_funds.argtypes, so.emu_short_funds.restype = [U, P, P, U, P, C.c_uint64, P], U
+    so.emu_write_overlap.argtypes = [P, P, U, P]
     return so
 
 
@@ -118,3 +119,16 @@ def test_transfers_without_funds_look_twice_behind_a_fence(emu, nr):
     bad = C.c_uint32()
     assert emu.emu_short_funds(nr, p(op), p(addr), 40, p(value), 1, C.byref(bad)) == 0xFFFFFFFF
     assert bad.value == 0
+
+
+def test_write_overlap_names_the_lower_lanes_with_a_common_address(emu):
+    rng = np.random.default_rng(4)
+    for case in range(40):
+        n_acc = int(rng.choice([2, 10, 64, 1000]))
+        ws, nws = rng.integers(0, n_acc, (32, 2)).astype(np.uint32), rng.integers(0, 3, 32).astype(np.uint32)
+        active = int(rng.integers(0, 1 << 32))
+        out = np.zeros(32, np.uint32)
+        emu.emu_write_overlap(p(ws), p(nws), active, p(out))
+        sets = [set(ws[l, :nws[l]].tolist()) if active >> l & 1 else set() for l in range(32)]
+        for l in range(32):
+            assert out[l] == sum(1 << i for i in range(l) if sets[i] & sets[l])

@@ -180,3 +180,16 @@ extern "C" uint32_t emu_short_funds(uint32_t nr, const uint32_t* op, const uint3
   emu::on_fence = [&] { open[emu::cur].clear(); };
   return emu::run(seed, 1ull << 24) ? fin : 0u;
 }
+
+// TXWriteOverlap of one warp: write sets ws [32][2] of nws[l] addresses.
+extern "C" void emu_write_overlap(const uint32_t* ws, const uint32_t* nws, uint32_t active, uint32_t* out) {
+  emu::reset();
+  emu::add_warp(0, 0, [&] {
+    const uint32_t l = lane_id();
+    WriteSet<2> x;
+    x.n = nws[l];
+    for (int k = 0; k < 2; k++) x.addr[k] = ws[2 * l + k];
+    out[l] = TXWriteOverlap(x, (active >> l) & 1u);
+  });
+  emu::run(1, 1ull << 20);
+}
