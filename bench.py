@@ -37,8 +37,8 @@ atomic rates of the GPU, the engine's roofline).
 
 --impl reference runs the reference arm: the path's CPU execution (the oracle port, striped
 locks on every host core) on the same batches, generated by the oracle's own generator.
---case NAME runs one small invocation of one kernel for profiling (engine, group, serial, flow,
-mlp, memcd, sched). Multi-GPU: replicas only (no collective on the path); each rank runs its own
+--case NAME runs one small invocation of one kernel for profiling (engine, group, uniform, serial,
+flow, mlp, grad, memcd, sched). Multi-GPU: replicas only (no collective on the path); each rank runs its own
 instance on its own GPU, value sums the ranks' transactions over the slowest rank's time.
 """
 from __future__ import annotations
@@ -84,7 +84,8 @@ def parse():
     ap.add_argument("--ctas", type=int, default=int(os.environ.get("CSMV_CTAS", 152)))
     ap.add_argument("--depth", type=int, default=int(os.environ.get("CSMV_DEPTH", 8)))
     ap.add_argument("--case", default=None,
-                    choices=["engine", "group", "serial", "flow", "mlp", "memcd", "sched"])
+                    choices=["engine", "group", "uniform", "serial", "flow", "mlp", "grad", "memcd",
+                             "sched"])
     ap.add_argument("--case-txn", type=int, default=1 << 18)
     ap.add_argument("--no-extras", action="store_true", help="skip the extra sections")
     ap.add_argument("--no-tune", action="store_true", help="skip the autotuner (use the flags)")
@@ -812,8 +813,8 @@ def run_case(args, local):
     import csmv_gb300 as cg
     torch.cuda.set_device(local)
     n = args.case_txn
-    if args.case in ("engine", "group", "serial", "flow", "sched"):
-        dist = "uniform" if args.case == "engine" else "zipf"
+    if args.case in ("engine", "group", "uniform", "serial", "flow", "sched"):
+        dist = "uniform" if args.case in ("engine", "uniform") else "zipf"
         s, bs = generate_batches(dist, n, 2, pinned=False)
         addr = torch.from_numpy(s.addr.view(np.int32)).cuda()
         dev = [DevBatch(torch, b) for b in bs]
@@ -827,22 +828,27 @@ def run_case(args, local):
             sched.close()
             out = {"case": args.case, "commits": r.commits, "planned_ms": r.planned.kernel_ms}
         else:
-            run = {"engine": bank.run_device, "serial": bank.run_serial_device,
-                   "flow": bank.run_flow_device}[args.case]
+            run = {"engine": bank.run_device, "uniform": bank.run_device,
+                   "serial": bank.run_serial_device, "flow": bank.run_flow_device}[args.case]
             for d in dev:  # a warm-up launch, then the profiled one
                 st = run(d.stream(cg, addr, s.addr.shape[0]))
             out = {"case": args.case, "commits": st.commits, "kernel_ms": st.kernel_ms}
         bank.close()
-    elif args.case == "mlp":
+    elif args.case in ("mlp", "grad"):
         rng = np.random.default_rng(0)
         x = (rng.random((n, 64)) < 0.2).astype(np.float32)
         bits = (x.view(np.uint32) >> 16).astype(np.uint16).view(np.int16)  # 0/1 exact in bf16
         dx = torch.from_numpy(bits).cuda()
         dp = torch.zeros(n, dtype=torch.float32, device="cuda")
+        dy = torch.from_numpy((rng.random(n) < 0.3).astype(np.float32)).cuda()
+        loss = None
         with cg.Mlp(seed=1, device=local) as m:
-            m.forward(n, dx.data_ptr(), dp.data_ptr())
-            m.forward(n, dx.data_ptr(), dp.data_ptr())
-        out = {"case": "mlp", "mean_p": float(dp.mean())}
+            for _ in range(2):  # a warm-up launch, then the profiled one
+                if args.case == "grad":
+                    loss = m.grad(n, dx.data_ptr(), dy.data_ptr())
+                else:
+                    m.forward(n, dx.data_ptr(), dp.data_ptr())
+        out = {"case": args.case, "loss": loss, "mean_p": float(dp.mean())}
     else:
         n = 1 << 16
         with cg.Memcd(n_sets=1 << 20, client_warps=4, max_req=n, log_commits=0, device=local) as c:
@@ -941,7 +947,8 @@ def main():
     tr = ROOT / "profiles" / "traffic.json"
     if tr.exists():
         try:
-            traffic = json.loads(tr.read_text()).get("bank_kernel_learned_bytes_per_launch")
+            traffic = json.loads(tr.read_text())["bank_kernel_learned_bytes_per_launch"].get(
+                f"{args.client_warps} client warps, depth {args.depth}")
         except Exception:
             traffic = None
     line = {

@@ -56,7 +56,7 @@ struct csmv_bank_t {
   uint32_t* d_lanes = nullptr;    // host-buffer runs: the stream's lanes of the deferred queue
   uint32_t* grp = nullptr;        // group-end bitmap of the last run (log_commits)
   uint32_t* tk = nullptr;         // group commit: per account {next ticket, ticket served}
-  int32_t* d_values = nullptr;    // balances of the last csmv_bank_read_values, copied out
+  int32_t* d_values = nullptr;    // balances on their way in (csmv_bank_load) or out (read_values)
   uint32_t grp_words = 0;
   bool last_grouped = false;      // the last run was a group-commit run of the engine
   uint64_t addr_cap = 0;

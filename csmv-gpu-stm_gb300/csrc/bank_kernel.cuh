@@ -839,7 +839,8 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
   //    lane writes any of its accounts to (every writer of an account also reads it, so two
   //    writers of one account are always dependent).
   //    When no lane's amount depends on a lower lane (the transfers read only their two
-  //    accounts, or move fixed amounts), the chain is a sum: each lane adds up the amounts the
+  //    accounts, or move fixed amounts: not those of csmv_bank_generate with extra reads, whose
+  //    amounts are drawn from the values read), the chain is a sum: each lane adds up the amounts the
   //    lower lanes move over its two accounts, assuming all of them move theirs. If then every
   //    lane's funds suffice, the assumption holds (by induction in lane order) and the values
   //    are the chain's; otherwise the walk below runs. That is 31 independent steps of one
@@ -1139,8 +1140,8 @@ __device__ uint32_t group_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm
 // waits point to smaller timestamps, so then someone commits whatever the others' timing is).
 // Bound by its chain of L2 round trips and fences (about 0.65 us a trip): loads that do not
 // depend on each other go out together, the victims' slots are read while the server draws, and
-// one pass over the candidates replaces the two all-pairs loops of TXWriteOverlap and
-// TXPreValidation (2.2 us).
+// one pass over the candidates finds what the all-pairs loops of TXWriteOverlap and
+// TXPreValidation (include/csmv_tx.cuh) find, which would take 2.2 us.
 template <int DEPTH, int MAXR, int MAXW, bool CLUSTER>
 __device__ uint32_t stamp_attempt(const BankParams& p, CtaShared<MAXR, MAXW>& sm,
                                   MailSlot<MAXR, MAXW>& ms, uint32_t me, uint32_t t, uint32_t op,

@@ -13,9 +13,10 @@
 // A writer (holding the entry's lock) empties the victim's tag, fences, writes the record,
 // fences and publishes the new tag; a reader re-reads the tag after the record, so a record is
 // used only if its tag did not move (a sequence-lock). The tags of a set's 8 ways sit in one
-// 128-byte line: a GET at snapshot S loads them in one access, picks per way the newest version
-// <= S, and reads only the records whose valid hash matches, in way order (first full key match
-// wins, as the reference breaks at the first match). A SET looks at each way's latest committed
+// 128-byte line: a GET reads the ways' commit words, takes each way's latest committed version
+// (the one its stamp names) from that line, and reads only the records whose valid hash matches,
+// in way order (first full key match wins, as the reference breaks at the first match). A SET
+// looks at each way's latest committed
 // version (by its commit word), chooses the slot by the reference's rule, locks only that entry,
 // takes a commit timestamp from the CTA's server, validates the eight stamps and installs the
 // new version. Rounds of 32 requests are warp-uniform GETs or SETs (memcdSH.cu:333-339).
@@ -23,9 +24,9 @@
 // Bound under Zipf(0.99) by the hottest entry's lock, through which its SETs pass one hold after
 // the other, and by the GETs that wait for holders. A warp's SETs of one key therefore share a
 // hold; a hold is kept to the timestamp draw, the validation and three fences; and records
-// are read only where a tag's hash says so. A batch of 64 K requests with 1 % SETs on 2^20 sets
-// took 2.3 ms before that and takes 0.21 ms; a serving session of 495 K requests with 5 % SETs
-// took 57 ms and takes 5.1 ms.
+// are read only where a tag's hash says so. A call of 64 K requests with 1 % SETs on a filled
+// table of 2^20 sets took 1.6 to 1.8 ms with one SET a hold and takes 0.24 to 0.27 ms; a serving
+// session of 495 K requests with 5 % SETs took 55 to 57 ms and takes 4.6 ms.
 #pragma once
 #include <cstdint>
 

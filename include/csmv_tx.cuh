@@ -216,9 +216,10 @@ __device__ __forceinline__ uint32_t TXPreValidation(const ReadSet<MAXR>& rs,
 }
 
 // Lanes below this one (among the active lanes) whose write sets share an address with this
-// lane's write set, warp-collective. The stamp protocol lets only the lowest writer of an
-// address in a warp try for its lock, so the warp's outcome never depends on which lane's atomic
-// the memory system serves first.
+// lane's write set, warp-collective. For callers that lock before they validate, as the stamp
+// protocol does: only the lowest writer of an address in a warp tries for its lock, so the warp's
+// outcome never depends on which lane's atomic the memory system serves first. (The engine finds
+// overlaps and conflicts in one pass of its own.)
 template <int MAXW>
 __device__ __forceinline__ uint32_t TXWriteOverlap(const WriteSet<MAXW>& ws, bool active) {
   const uint32_t me = lane_id();
