@@ -247,7 +247,6 @@ bool csmv::flow_serial_run(csmv_bank_t* h, const csmv_bank_stream* s, csmv_stats
   *st = flow_run(h, s, spin, &stats, &ready);
   if (*st != CSMV_OK && !ready) {
     if (*st == CSMV_ERR_CAPACITY) return false;  // too many accesses: the buffers are in order
-    cudaGetLastError();  // an allocation that failed is no error of the next launch
     flow_scratch_free(h->flow);
     h->flow = nullptr;
     return false;

@@ -11,9 +11,12 @@ namespace csmv {
 
 void set_error(const char* fmt, ...) __attribute__((format(printf, 1, 2)));
 
-// Record a CUDA failure and turn it into a status (never aborts the process).
+// Record a CUDA failure and turn it into a status (never aborts the process). The runtime keeps a
+// failure until it is asked for its last error: it is taken back here, so that a refused call (an
+// allocation, say) is not reported once more by the check behind the next kernel launch.
 inline csmv_status cuda_status(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return CSMV_OK;
+  cudaGetLastError();
   set_error("%s: %s", what, cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? CSMV_ERR_OOM : CSMV_ERR_CUDA;
 }

@@ -5,6 +5,7 @@ order reproduces the device's final version slots bit for bit, every read-only a
 transaction saw the state at its snapshot, commit timestamps are unique and dense, the total
 balance is conserved. With one client warp the run is deterministic and must equal the oracle's
 model of the engine exactly (log, outcomes, versions, abort counts)."""
+import ctypes as C
 import subprocess
 
 import numpy as np
@@ -840,3 +841,17 @@ def test_streams_of_few_rounds_in_every_commit_mode(mode, rounds):
     run_checked(c1_workload(n_txn=32 * rounds, n_accounts=512, up_reads=3, pr_read_pct=20, seed=rounds),
                 ctas=3, client_warps=4, validate=validate, writeback=writeback, batch=batch,
                 prevalidate=prevalidate)
+
+
+def test_a_refused_allocation_is_no_error_of_the_next_call():
+    """An allocation that is refused (2^50 bytes of host memory) fails its own call; loading a bank,
+    running it and reading it back on the same thread then work as ever."""
+    ptr = C.c_void_p()
+    assert cg.lib().csmv_pinned_alloc(C.c_size_t(1 << 50), C.byref(ptr)) != 0
+    w = c1_workload(n_txn=32 * 8, n_accounts=64)
+    s = cg.generate(w)
+    with cg.Bank(n_accounts=64, max_txn=w.n_txn) as bank:
+        for step in (bank.load, lambda: bank.run(s), bank.values):
+            assert cg.lib().csmv_pinned_alloc(C.c_size_t(1 << 50), C.byref(ptr)) != 0
+            step()
+        assert bank.values().sum() == 64 * 1000
