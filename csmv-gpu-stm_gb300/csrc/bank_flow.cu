@@ -221,7 +221,11 @@ csmv_status flow_run(csmv_bank_t* h, const csmv_bank_stream* s, uint32_t spin_lo
                      bool* ready) {
   *ready = false;
   csmv_status st = ensure_txn(h, s->n_txn);
-  if (st != CSMV_OK) return st;
+  if (st != CSMV_OK) {  // no half-made buffers for the next run
+    flow_scratch_free(h->flow);
+    h->flow = nullptr;
+    return st;
+  }
   h->last_grouped = false;  // the lane installs every write
   if ((st = bank_begin_run(h)) != CSMV_OK) return st;
   csmv_status lst = flow_launch(h, s, spin_log2, ready);
